@@ -151,6 +151,44 @@ __device__ __forceinline__ int quant_lane(float v, __half* d_out) {
     return q;
 }
 
+// quant_lane for four neighbouring values per thread: eight threads (t = lane % 8) hold a 32-block, element 4t + j in v[j].
+// The butterfly is quant_lane's step by step (strides 16, 8, 4 across threads, 2 and 1 across j), so that a block with
+// NaNs, where the maximum differs from element to element, gives the same bytes too.  d_out is element 0's (t = 0).
+__device__ __forceinline__ char4 quant_four(const float (&v)[4], __half* d_out) {
+    float a[4];
+#pragma unroll
+    for (int j = 0; j < 4; j++) a[j] = fabsf(v[j]);
+#pragma unroll
+    for (int s = 4; s > 0; s >>= 1)
+#pragma unroll
+        for (int j = 0; j < 4; j++) {
+            const float o = __shfl_xor_sync(0xffffffffu, a[j], s);
+            if (o > a[j]) a[j] = o;
+        }
+#pragma unroll
+    for (int s = 2; s > 0; s >>= 1) {
+        float n[4];
+#pragma unroll
+        for (int j = 0; j < 4; j++) n[j] = a[j ^ s] > a[j] ? a[j ^ s] : a[j];
+#pragma unroll
+        for (int j = 0; j < 4; j++) a[j] = n[j];
+    }
+    const bool same = a[0] == a[1] && a[0] == a[2] && a[0] == a[3];
+    int q[4];
+    float dq = 0.0f;
+#pragma unroll
+    for (int j = 0; j < 4; j++) {
+        if (j == 0 || !same) {
+            const __half dh = __float2half_rn((a[j] > 0.0f) ? __fdiv_rn(a[j], 127.0f) : 1.0f);
+            if (j == 0) *d_out = dh;
+            dq = __half2float(dh);
+        }
+        q[j] = (int)rintf(__fdiv_rn(v[j], dq));
+        q[j] = q[j] < -127 ? -127 : (q[j] > 127 ? 127 : q[j]);
+    }
+    return make_char4((signed char)q[0], (signed char)q[1], (signed char)q[2], (signed char)q[3]);
+}
+
 __device__ __forceinline__ float silu_mul(float g, float u) {
     return __fmul_rn(__fdiv_rn(g, __fadd_rn(1.0f, expf(-g))), u);
 }

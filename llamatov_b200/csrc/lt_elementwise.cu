@@ -8,8 +8,25 @@
 namespace lt {
 
 // ------------------------------------------------------------------ quantiser
-// one warp per 32-block, lane = element
+// Four elements per thread: bound by the bytes (5 per element) once there are enough of them; a warp per block, one
+// element per lane (k_quant_q8_any, any alignment), issued four times the loads and stores and twice the divisions
+// (2048 x 4864: 29.6 us, now 18.5 us; 2048 x 896: 8.3, now 5.3).
 __global__ void __launch_bounds__(256) k_quant_q8(const float* __restrict__ X, int8_t* __restrict__ Xq,
+                                                  __half* __restrict__ Xd, long nblocks) {
+    const long i = (long)blockIdx.x * 256 + threadIdx.x;      // quad of elements
+    const long b = i >> 3;
+    const bool ok = b < nblocks;
+    const float4 x = ok ? ((const float4*)X)[i] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    const float v[4] = {x.x, x.y, x.z, x.w};
+    __half dh;
+    const char4 q = quant_four(v, &dh);
+    if (!ok) return;
+    if ((i & 7) == 0) Xd[b] = dh;
+    ((char4*)Xq)[i] = q;
+}
+
+// one warp per 32-block, lane = element
+__global__ void __launch_bounds__(256) k_quant_q8_any(const float* __restrict__ X, int8_t* __restrict__ Xq,
                                                    __half* __restrict__ Xd, long nblocks) {
     long b = (long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
     int lane = threadIdx.x & 31;
@@ -288,8 +305,10 @@ extern "C" int lt_quant_q8(const float* X, int8_t* Xq, uint16_t* Xd, int K, int 
     LT_REQUIRE(X && Xq && Xd, "lt_quant_q8: null pointer");
     LT_REQUIRE(K > 0 && K % 32 == 0 && rows > 0, "lt_quant_q8: K=%d must be a positive multiple of 32, rows=%d > 0", K, rows);
     long nblocks = (long)rows * (K / 32);
-    unsigned grid = (unsigned)((nblocks + 7) / 8);
-    k_quant_q8<<<grid, 256, 0, (cudaStream_t)stream>>>(X, Xq, (__half*)Xd, nblocks);
+    if (aligned16(X) && (reinterpret_cast<uintptr_t>(Xq) & 3u) == 0)
+        k_quant_q8<<<(unsigned)((nblocks + 31) / 32), 256, 0, (cudaStream_t)stream>>>(X, Xq, (__half*)Xd, nblocks);
+    else
+        k_quant_q8_any<<<(unsigned)((nblocks + 7) / 8), 256, 0, (cudaStream_t)stream>>>(X, Xq, (__half*)Xd, nblocks);
     return check_launch("lt_quant_q8");
 }
 

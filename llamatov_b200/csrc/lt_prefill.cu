@@ -76,7 +76,28 @@ __global__ void k_add_len(int* len, int n, int max_seq) {
 }
 
 // ------------------------------------------------------------------ silu * up -> quant, strided rows
-__global__ void k_silu_mul_quant_rows(const float* __restrict__ G, const float* __restrict__ U, int ld,
+// Four elements per thread, eight threads per block: bound by its 9 bytes per element and by the exponential and the
+// divisions of silu and the quantiser.  A warp per block with one element per lane (k_silu_mul_quant_rows_any, any
+// alignment) had four times the instructions around them: 2048 rows of 4864, 53.7 us, now 28.7 us.
+__global__ void __launch_bounds__(256) k_silu_mul_quant_rows(const float* __restrict__ G, const float* __restrict__ U, int ld,
+                                                             int8_t* __restrict__ Xq, __half* __restrict__ Xd, int K, int rows) {
+    chain_release();
+    chain_wait();
+    const unsigned quads = (unsigned)K >> 2;
+    const long i = (long)blockIdx.x * 256 + threadIdx.x;      // quad of elements, row-major
+    const bool ok = i < (long)rows * quads;
+    const long r = ok ? i / quads : 0;
+    const long src = r * ld + (ok ? i - r * quads : 0) * 4;
+    const float4 g = *(const float4*)(G + src), u = *(const float4*)(U + src);
+    const float v[4] = {silu_mul(g.x, u.x), silu_mul(g.y, u.y), silu_mul(g.z, u.z), silu_mul(g.w, u.w)};
+    __half d;
+    const char4 q = quant_four(v, &d);
+    if (!ok) return;
+    ((char4*)Xq)[i] = q;
+    if ((i & 7) == 0) Xd[i >> 3] = d;
+}
+
+__global__ void k_silu_mul_quant_rows_any(const float* __restrict__ G, const float* __restrict__ U, int ld,
                                       int8_t* __restrict__ Xq, __half* __restrict__ Xd, int K, int rows) {
     chain_release();
     chain_wait();
@@ -571,8 +592,12 @@ extern "C" int lt_silu_mul_quant_rows(const float* g, const float* u, int ld, in
     LT_REQUIRE(g && u && Xq && Xd, "lt_silu_mul_quant_rows: null pointer");
     LT_REQUIRE(K > 0 && K % 32 == 0 && rows > 0 && ld >= K, "lt_silu_mul_quant_rows: K=%d rows=%d ld=%d", K, rows, ld);
     const long blocks32 = (long)rows * (K / 32);
-    const cudaError_t e = launch_chained(k_silu_mul_quant_rows, dim3((unsigned)((blocks32 + 7) / 8)), dim3(256), 0,
-                                         (cudaStream_t)stream, g, u, ld, Xq, (__half*)Xd, K, rows);
+    const bool quads = aligned16(g) && aligned16(u) && ld % 4 == 0 && (reinterpret_cast<uintptr_t>(Xq) & 3u) == 0;
+    const cudaError_t e =
+        quads ? launch_chained(k_silu_mul_quant_rows, dim3((unsigned)((blocks32 + 31) / 32)), dim3(256), 0, (cudaStream_t)stream, g, u,
+                               ld, Xq, (__half*)Xd, K, rows)
+              : launch_chained(k_silu_mul_quant_rows_any, dim3((unsigned)((blocks32 + 7) / 8)), dim3(256), 0, (cudaStream_t)stream, g, u,
+                               ld, Xq, (__half*)Xd, K, rows);
     return check_launch("lt_silu_mul_quant_rows", 1, e);
 }
 

@@ -44,6 +44,36 @@ def test_quant_batched_rows(oracle):
         assert np.array_equal(host(xd, np.uint16).reshape(5, -1)[r], od.view(np.uint16))
 
 
+@pytest.mark.parametrize("K,rows", [(32, 1), (32, 31), (96, 33), (896, 5)])
+def test_quantisers_of_four_elements_per_thread(K, rows):
+    """The vector forms give the bytes of the lane-per-element forms (taken for addresses off the 16-byte grid), with
+    NaNs, infinities and blocks of zeros among the values."""
+    rng = np.random.default_rng(K + rows)
+    n = rows * K
+
+    def values():
+        x = rng.standard_normal(n).astype(np.float32)
+        x[:32] = 0.0
+        for i, v in enumerate((np.nan, np.inf, -np.inf, np.nan)):
+            x[(37 * i + 5) % n] = v
+        return x
+    g, u = values(), values()
+
+    def run(shift):
+        dg, du = torch.zeros(n + 4, device="cuda"), torch.zeros(n + 4, device="cuda")
+        dg[shift:shift + n], du[shift:shift + n] = torch.from_numpy(g).cuda(), torch.from_numpy(u).cuda()
+        out = []
+        for call in (lambda xq, xd: _lib.call("lt_quant_q8", dg[shift:].data_ptr(), xq, xd, K, rows, stream()),
+                     lambda xq, xd: _lib.call("lt_silu_mul_quant_rows", dg[shift:].data_ptr(), du[shift:].data_ptr(), K, xq, xd, K, rows, stream())):
+            xq = torch.full((n,), 99, dtype=torch.int8, device="cuda")
+            xd = torch.zeros(n // 32, dtype=torch.int16, device="cuda")
+            call(xq.data_ptr(), xd.data_ptr())
+            out += [host(xq), host(xd)]
+        return out
+    for a, b in zip(run(0), run(1)):
+        assert np.array_equal(a, b)
+
+
 def test_silu_mul_quant(oracle):
     rng = np.random.default_rng(6)
     K = 4864
