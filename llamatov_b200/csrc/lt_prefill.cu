@@ -506,6 +506,254 @@ static int launch_attn_prefill_wide(const float* Q, int q_ld, const float* K, co
     return check_launch("lt_attn_prefill");
 }
 
+// ---- the same attention for long chunks: 32 query rows per CTA of 128 threads, as register-blocked products over tiles
+// of 64 positions.  A score is a chain over d and an output a chain over positions, but different scores and outputs are
+// independent, so both are halves of a blocked fp32 product whose inner loop runs in the declared order.  What the
+// 16-row form above spends its time on is operand reads (6 of 16 bytes per 32 multiply-adds, 256 of 512 threads
+// folding, one CTA per SM, phases between barriers).  Here a thread owns 4 rows x 4 positions, then 4 rows x HD / 16
+// elements: 8 reads, 4 of them nearly broadcasts, per 64 multiply-adds, and four CTAs overlap on an SM.  Scores are
+// computed twice, first for the row maxima alone: no SM holds 32 rows of scores beside the tiles, and nothing depends
+// on Lmax.  A row's 64 softmax lanes are the 64 positions of a tile, so the lane sums of the denominator stay in the
+// registers of the threads that make the probabilities.  Bound by the multiply-adds (three products of Lmax^2 / 2 x
+// HD per head) and by the uneven lengths of the rows.
+// 2048 positions: 14 heads on 2 of 64: 505 us with 16 rows, now 350; 32 heads on 8 of 128: 3273, now 1549.
+// (64 rows per CTA, 8 x 4 per thread: 444; the 448 CTAs are all resident at once and share the SMs unevenly.)
+constexpr int PB_TILE = 64;
+
+template <int HD, int QT>
+struct PrefillBlock {
+    static constexpr int THREADS = 128;
+    static constexpr int ST = HD + 4;                    // floats between rows: conflict-free 16-byte reads
+    static constexpr int PST = PB_TILE + 4;
+    static constexpr int SMEM = (QT * ST + 2 * PB_TILE * ST + QT * PST + QT) * 4;
+};
+
+template <int HD, int QT>
+__global__ void __launch_bounds__(PrefillBlock<HD, QT>::THREADS)
+k_attn_prefill_block(const float* __restrict__ Q, int q_ld, const float* __restrict__ K, const float* __restrict__ V,
+                     const int* __restrict__ len_ptr, float* __restrict__ OUT, int out_ld, int nh, int nkv, float scale,
+                     int nrows, int maxt, int* status) {
+    using B = PrefillBlock<HD, QT>;
+    constexpr int PB_THREADS = B::THREADS, ST = B::ST, PST = B::PST, MQ = QT * 16 / PB_THREADS, ND = HD / 64;
+    extern __shared__ __align__(16) float pf_smem[];
+    float* qs = pf_smem;                     // [QT][ST]
+    float* tk = qs + QT * ST;                // [PB_TILE][ST]  K
+    float* tv = tk + PB_TILE * ST;           // [PB_TILE][ST]  V (the other K buffer while the maxima are found)
+    float* ps = tv + PB_TILE * ST;           // [QT][PST] probabilities of a tile, at the end the lane sums
+    float* zs = ps + QT * PST;               // [QT]
+    const int tid = threadIdx.x, n = tid & 15, m = tid >> 4;
+    const int h = blockIdx.x % nh;
+    const int r0 = ((int)gridDim.x / nh - 1 - (int)blockIdx.x / nh) * QT;     // the longest rows first
+    const int Lafter = *len_ptr;
+    if (Lafter < nrows || Lafter > maxt) {
+        if (tid == 0) atomicOr(status, (int)LT_STATUS_BAD_LENGTH);
+        return;
+    }
+    const int L0 = Lafter - nrows;
+    const int nq = nrows - r0 < QT ? nrows - r0 : QT;
+    const int Lmax = L0 + r0 + nq;
+    const int hk = h / (nh / nkv);
+    const long rstride = (long)nkv * HD;
+
+    auto copy_tile = [&](const float* base, int t0, float* dst) {     // positions [t0, t0 + 64) of head hk; zeros from Lmax on
+        const float* src = base + (long)hk * HD + (long)t0 * rstride;
+#pragma unroll 4
+        for (int e = tid; e < PB_TILE * (HD / 4); e += PB_THREADS) {
+            const int r = e / (HD / 4), c = e - r * (HD / 4);
+            const bool ok = t0 + r < Lmax;
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"((unsigned)__cvta_generic_to_shared(dst + r * ST + c * 4)),
+                         "l"(ok ? src + (long)r * rstride + c * 4 : base), "r"(ok ? 16 : 0)
+                         : "memory");
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    // scores of rows m * MQ + i and positions t0 + n + 16 j of a K tile, not yet scaled
+    auto scores = [&](const float* kt, float (&s)[MQ][4]) {
+#pragma unroll
+        for (int i = 0; i < MQ; i++)
+#pragma unroll
+            for (int j = 0; j < 4; j++) s[i][j] = 0.0f;
+        const float4* K4 = (const float4*)(kt + n * ST);
+        const float4* Q4 = (const float4*)(qs + m * MQ * ST);
+#pragma unroll 4
+        for (int d = 0; d < HD / 4; d++) {
+            float4 k[4], q[MQ];
+#pragma unroll
+            for (int j = 0; j < 4; j++) k[j] = K4[j * 16 * (ST / 4) + d];
+#pragma unroll
+            for (int i = 0; i < MQ; i++) q[i] = Q4[i * (ST / 4) + d];
+#pragma unroll
+            for (int i = 0; i < MQ; i++)
+#pragma unroll
+                for (int j = 0; j < 4; j++) s[i][j] = __fmaf_rn(q[i].x, k[j].x, s[i][j]);
+#pragma unroll
+            for (int i = 0; i < MQ; i++)
+#pragma unroll
+                for (int j = 0; j < 4; j++) s[i][j] = __fmaf_rn(q[i].y, k[j].y, s[i][j]);
+#pragma unroll
+            for (int i = 0; i < MQ; i++)
+#pragma unroll
+                for (int j = 0; j < 4; j++) s[i][j] = __fmaf_rn(q[i].z, k[j].z, s[i][j]);
+#pragma unroll
+            for (int i = 0; i < MQ; i++)
+#pragma unroll
+                for (int j = 0; j < 4; j++) s[i][j] = __fmaf_rn(q[i].w, k[j].w, s[i][j]);
+        }
+    };
+
+    copy_tile(K, 0, tk);
+    for (int e = tid; e < QT * (HD / 4); e += PB_THREADS) {
+        const int r = e / (HD / 4), c = e - r * (HD / 4);
+        *(float4*)(qs + r * ST + c * 4) =
+            r < nq ? *(const float4*)(Q + (long)(r0 + r) * q_ld + (long)h * HD + c * 4) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    }
+    int lim[MQ];                             // positions that row i sees
+#pragma unroll
+    for (int i = 0; i < MQ; i++) lim[i] = L0 + r0 + m * MQ + i + 1;
+
+    // ---- row maxima
+    float mx[MQ];
+#pragma unroll
+    for (int i = 0; i < MQ; i++) mx[i] = -1e30f;
+    for (int t0 = 0, buf = 0; t0 < Lmax; t0 += PB_TILE, buf ^= 1) {
+        if (t0 + PB_TILE < Lmax) {
+            copy_tile(K, t0 + PB_TILE, buf ? tk : tv);
+            asm volatile("cp.async.wait_group 1;" ::: "memory");
+        } else {
+            asm volatile("cp.async.wait_group 0;" ::: "memory");
+        }
+        __syncthreads();
+        float s[MQ][4];
+        scores(buf ? tv : tk, s);
+#pragma unroll
+        for (int i = 0; i < MQ; i++)
+#pragma unroll
+            for (int j = 0; j < 4; j++)
+                if (t0 + n + 16 * j < lim[i]) mx[i] = fmaxf(mx[i], __fmul_rn(s[i][j], scale));
+        __syncthreads();
+    }
+    copy_tile(K, 0, tk);
+    copy_tile(V, 0, tv);
+#pragma unroll
+    for (int i = 0; i < MQ; i++)
+#pragma unroll
+        for (int x = 8; x > 0; x >>= 1) mx[i] = fmaxf(mx[i], __shfl_xor_sync(0xffffffffu, mx[i], x));
+
+    // ---- probabilities, lane sums of the denominator, V sum
+    float z[MQ][4], acc[ND][MQ][4];
+#pragma unroll
+    for (int i = 0; i < MQ; i++)
+#pragma unroll
+        for (int j = 0; j < 4; j++) {
+            z[i][j] = 0.0f;
+#pragma unroll
+            for (int g = 0; g < ND; g++) acc[g][i][j] = 0.0f;
+        }
+    for (int t0 = 0; t0 < Lmax; t0 += PB_TILE) {
+        const bool more = t0 + PB_TILE < Lmax;
+        asm volatile("cp.async.wait_group 1;" ::: "memory");      // K of this tile; V may be on its way
+        __syncthreads();
+        {
+            float s[MQ][4];
+            scores(tk, s);
+#pragma unroll
+            for (int i = 0; i < MQ; i++)
+#pragma unroll
+                for (int j = 0; j < 4; j++) {
+                    const float e = t0 + n + 16 * j < lim[i] ? __expf(__fsub_rn(__fmul_rn(s[i][j], scale), mx[i])) : 0.0f;
+                    z[i][j] = __fadd_rn(z[i][j], e);
+                    ps[(m * MQ + i) * PST + n + 16 * j] = e;
+                }
+        }
+        asm volatile("cp.async.wait_group 0;" ::: "memory");
+        __syncthreads();                                          // probabilities and V are there, K may be replaced
+        if (more) copy_tile(K, t0 + PB_TILE, tk);
+        const float* pr = ps + m * MQ * PST;
+        if (t0 + PB_TILE <= L0 + r0 + 1) {                        // every row sees the whole tile
+#pragma unroll 2
+            for (int t = 0; t < PB_TILE; t += 4) {
+                float4 p[MQ];
+#pragma unroll
+                for (int i = 0; i < MQ; i++) p[i] = *(const float4*)(pr + i * PST + t);
+#pragma unroll
+                for (int g = 0; g < ND; g++) {
+                    float4 v[4];
+#pragma unroll
+                    for (int j = 0; j < 4; j++) v[j] = *(const float4*)(tv + (t + j) * ST + g * 64 + n * 4);
+#pragma unroll
+                    for (int j = 0; j < 4; j++)
+#pragma unroll
+                        for (int i = 0; i < MQ; i++) {
+                            const float w = j == 0 ? p[i].x : (j == 1 ? p[i].y : (j == 2 ? p[i].z : p[i].w));
+                            acc[g][i][0] = __fmaf_rn(w, v[j].x, acc[g][i][0]);
+                            acc[g][i][1] = __fmaf_rn(w, v[j].y, acc[g][i][1]);
+                            acc[g][i][2] = __fmaf_rn(w, v[j].z, acc[g][i][2]);
+                            acc[g][i][3] = __fmaf_rn(w, v[j].w, acc[g][i][3]);
+                        }
+                }
+            }
+        } else {                                                  // the causal edge: a row stops at its own position
+            const int te = more ? PB_TILE : Lmax - t0;
+            for (int t = 0; t < te; t++) {
+#pragma unroll
+                for (int g = 0; g < ND; g++) {
+                    const float4 v = *(const float4*)(tv + t * ST + g * 64 + n * 4);
+#pragma unroll
+                    for (int i = 0; i < MQ; i++)
+                        if (t0 + t < lim[i]) {
+                            const float w = pr[i * PST + t];
+                            acc[g][i][0] = __fmaf_rn(w, v.x, acc[g][i][0]);
+                            acc[g][i][1] = __fmaf_rn(w, v.y, acc[g][i][1]);
+                            acc[g][i][2] = __fmaf_rn(w, v.z, acc[g][i][2]);
+                            acc[g][i][3] = __fmaf_rn(w, v.w, acc[g][i][3]);
+                        }
+                }
+            }
+        }
+        __syncthreads();                                          // V and the probabilities may be replaced
+        if (more) copy_tile(V, t0 + PB_TILE, tv);
+    }
+
+    // ---- denominator: 64 lanes of a row, then the tree
+#pragma unroll
+    for (int i = 0; i < MQ; i++)
+#pragma unroll
+        for (int j = 0; j < 4; j++) ps[(m * MQ + i) * PST + n + 16 * j] = z[i][j];
+    __syncthreads();
+    for (int r = tid >> 5; r < QT; r += PB_THREADS / 32) {
+        const float v = warp_tree_sum(__fadd_rn(ps[r * PST + (tid & 31)], ps[r * PST + (tid & 31) + 32]));
+        if ((tid & 31) == 0) zs[r] = v;
+    }
+    __syncthreads();
+#pragma unroll
+    for (int i = 0; i < MQ; i++) {
+        const int r = m * MQ + i;
+        if (r >= nq) continue;
+        const float zr = zs[r];
+#pragma unroll
+        for (int g = 0; g < ND; g++) {
+            float* o = OUT + (long)(r0 + r) * out_ld + (long)h * HD + g * 64 + n * 4;
+            ((float2*)o)[0] = make_float2(__fdiv_rn(acc[g][i][0], zr), __fdiv_rn(acc[g][i][1], zr));
+            ((float2*)o)[1] = make_float2(__fdiv_rn(acc[g][i][2], zr), __fdiv_rn(acc[g][i][3], zr));
+        }
+    }
+}
+
+template <int HD, int QT>
+static int launch_attn_prefill_block(const float* Q, int q_ld, const float* K, const float* V, const int* len, float* OUT,
+                                     int out_ld, int nh, int nkv, float scale, int nrows, int maxt, cudaStream_t s) {
+    int* st = device_status_ptr();
+    LT_REQUIRE(st != nullptr, "lt_attn_prefill: status word unavailable");
+    constexpr int smem = PrefillBlock<HD, QT>::SMEM;
+    static PerDeviceOnce attr_once;
+    if (attr_once.first()) {
+        LT_CUDA(cudaFuncSetAttribute(k_attn_prefill_block<HD, QT>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+    }
+    k_attn_prefill_block<HD, QT><<<(nrows + QT - 1) / QT * nh, PrefillBlock<HD, QT>::THREADS, smem, s>>>(Q, q_ld, K, V, len, OUT, out_ld,
+                                                                                                        nh, nkv, scale, nrows, maxt, st);
+    return check_launch("lt_attn_prefill");
+}
+
 template <int HD, int QT>
 static int launch_attn_prefill(const float* Q, int q_ld, const float* K, const float* V, const int* len, float* OUT,
                                int out_ld, int nh, int nkv, float scale, int nrows, int maxt, cudaStream_t s) {
@@ -527,12 +775,17 @@ static int launch_attn_prefill(const float* Q, int q_ld, const float* K, const f
 template <int HD>
 static int pick_attn_prefill(const float* Q, int q_ld, const float* K, const float* V, const int* len, float* OUT,
                              int out_ld, int nh, int nkv, float scale, int nrows, int maxt, cudaStream_t s) {
+    if (nrows >= 32 && aligned16(V)) {
+        // 32 rows per CTA from three CTAs per SM on: 1000 rows of 14 heads (448 CTAs) take 147 us either way; below,
+        // smaller tiles fill the SMs better (333 rows: 31 us with 16 rows per CTA, 39 with 32) ...
+        if ((long)((nrows + 31) / 32) * nh >= 448)
+            return launch_attn_prefill_block<HD, 32>(Q, q_ld, K, V, len, OUT, out_ld, nh, nkv, scale, nrows, maxt, s);
+        // ... where the score rows of 16 queries fit one SM beside double-buffered tiles
+        if (attn_prefill_wide_smem<HD>(maxt) <= 227 * 1024)
+            return launch_attn_prefill_wide<HD>(Q, q_ld, K, V, len, OUT, out_ld, nh, nkv, scale, nrows, maxt, s);
+    }
     // query rows per tile: 8 while three CTAs of score rows fit an SM (the V sum and the softmax are
-    // chains of dependent operations, resident warps hide them), else 4; 16 only for short chunks (16 rows
-    // with one CTA per SM was measured 6 % slower at 2048 positions)
-    // 16 rows per CTA with double-buffered tiles where the score rows of 16 queries fit one SM beside them
-    if (nrows >= 2 * PW_QT && attn_prefill_wide_smem<HD>(maxt) <= 227 * 1024 && aligned16(V))
-        return launch_attn_prefill_wide<HD>(Q, q_ld, K, V, len, OUT, out_ld, nh, nkv, scale, nrows, maxt, s);
+    // chains of dependent operations, resident warps hide them), else 4; 16 only for short chunks
     const size_t per_row = (size_t)((maxt + 3) & ~3) + HD + 65;
     const size_t tile = (size_t)PF_KTILE * (HD + 4) * sizeof(float);
     if (16 * per_row * sizeof(float) + tile <= 72 * 1024)

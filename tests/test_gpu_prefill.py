@@ -167,3 +167,29 @@ def test_chunk_attention_equals_one_token_attention(hd, nh, nkv):
                   one.data_ptr(), hd, nh, nkv, scale, maxseq, stream())
         assert np.array_equal(bits(got[r]), bits(host(one))), r
     assert _lib.device_status() == set()
+
+
+@pytest.mark.parametrize("hd,nh,nkv,L0,T", [(64, 14, 2, 0, 993), (64, 56, 8, 63, 257), (64, 64, 4, 5, 224), (128, 32, 8, 0, 449), (128, 64, 8, 130, 193)])
+def test_attention_of_long_chunks_equals_one_token_attention(hd, nh, nkv, L0, T):
+    """Enough rows and heads for 32 rows per CTA: whole and ragged row tiles, tiles of positions cut by the chunk's start."""
+    rng = np.random.default_rng(T)
+    maxseq, width = L0 + T + 9, nkv * hd
+    K = (rng.standard_normal((maxseq, width)) * 0.5).astype(np.float32)
+    V = rng.standard_normal((maxseq, width)).astype(np.float32)
+    K[L0 + T:] = np.nan; V[L0 + T:] = np.nan
+    V[L0 + T - 1] = np.inf                             # only the last row may see it
+    Q = rng.standard_normal((T, nh * hd)).astype(np.float32)
+    dK, dV, dQ = dev(K.reshape(-1)), dev(V.reshape(-1)), dev(Q.reshape(-1))
+    scale = float(np.float32(hd ** -0.5))
+    out = torch.full((T * nh * hd,), float("nan"), device="cuda")
+    ln = torch.tensor([L0 + T], dtype=torch.int32, device="cuda")
+    _lib.call("lt_attn_prefill", dQ.data_ptr(), nh * hd, dK.data_ptr(), dV.data_ptr(), ln.data_ptr(), out.data_ptr(),
+              nh * hd, hd, nh, nkv, scale, T, L0 + T, stream())
+    got = host(out).reshape(T, nh * hd)
+    one = torch.empty(nh * hd, device="cuda")
+    for r in sorted({0, 1, 31, 32, 63, 64, T // 2, T - 33, T - 2, T - 1}):
+        ln1 = torch.tensor([L0 + r + 1], dtype=torch.int32, device="cuda")
+        _lib.call("lt_attn_decode_masked", dQ[r * nh * hd:].data_ptr(), dK.data_ptr(), dV.data_ptr(), ln1.data_ptr(),
+                  one.data_ptr(), hd, nh, nkv, scale, maxseq, stream())
+        assert np.array_equal(bits(got[r]), bits(host(one))), r
+    assert _lib.device_status() == set()
