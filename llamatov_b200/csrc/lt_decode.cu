@@ -110,6 +110,13 @@ __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wai
 
 __device__ __forceinline__ void consumer_sync() { asm volatile("bar.sync 1, %0;" ::"n"(DEC_CTHREADS) : "memory"); }
 __device__ __forceinline__ void pair_sync() { asm volatile("bar.sync 2, 64;" ::: "memory"); }   // warps 0 and 1
+// Segments of cached V rows (attention CTA): buffer b of four is full / free.  Warps 0 and 1 fold, warps V_COPIERS_FROM.. copy.
+constexpr int V_COPIERS_FROM = 3;
+constexpr int V_PARTIES = 64 + DEC_CTHREADS - V_COPIERS_FROM * 32;
+__device__ __forceinline__ void v_segment_full_arrive(int b) { asm volatile("bar.arrive %0, %1;" ::"r"(4 + b), "n"(V_PARTIES) : "memory"); }
+__device__ __forceinline__ void v_segment_full_wait(int b) { asm volatile("bar.sync %0, %1;" ::"r"(4 + b), "n"(V_PARTIES) : "memory"); }
+__device__ __forceinline__ void v_segment_free_arrive(int b) { asm volatile("bar.arrive %0, %1;" ::"r"(8 + b), "n"(V_PARTIES) : "memory"); }
+__device__ __forceinline__ void v_segment_free_wait(int b) { asm volatile("bar.sync %0, %1;" ::"r"(8 + b), "n"(V_PARTIES) : "memory"); }
 
 // tagged element: {payload, tag} in one 8-byte word
 __device__ __forceinline__ void st_tagged(float2* p, float v, unsigned tag) { __stcg(p, make_float2(v, __uint_as_float(tag))); }
@@ -815,7 +822,14 @@ __device__ __forceinline__ void attention_layer(const lt_decode_desc& P, const l
     }
     const int L = room ? pos + 1 : pos;      // attention length after the append
     const int Lc = room ? pos : L;           // rows that already live in the cache
-    const int vst = Lc < vcap ? Lc : vcap;   // cached V rows staged in shared memory
+    // Cached V rows are staged in shared memory.  A context with more rows than fit goes through it in segments of seg
+    // rows, four buffers: the first four now, the others during the V fold, each when the one four before it is folded
+    // (warps 3.. copy, warps 0 and 1 fold).  Folding the rest from global memory, eight rows per round trip to L2, cost
+    // more than the whole rest of the layer: 1000 positions 1178 us per token, now 811 us (32 positions: 376).
+    const int seg = vcap / 16 * 4;
+    const bool in_segments = Lc > vcap && seg > 0;
+    const int nseg = in_segments ? (Lc + seg - 1) / seg : 0;
+    const int vst = Lc <= vcap ? Lc : (in_segments ? 4 * seg : vcap);
 
     // ---- before the layer input is awaited: everything that does not depend on it
     // cached K rows in registers: position tid/2, the even thread holds the first half of the row,
@@ -923,7 +937,7 @@ __device__ __forceinline__ void attention_layer(const lt_decode_desc& P, const l
                                               : (const float4*)(ly->kcache + ((size_t)t * nkv + hk) * HD);
         const float4* q4 = (const float4*)A.q;
         float s = 0.0f;
-#pragma unroll 4
+#pragma unroll 8
         for (int i = 0; i < HD4; i++) {
             const float4 qq = q4[i], kk = k4[i];
             s = __fmaf_rn(qq.x, kk.x, s); s = __fmaf_rn(qq.y, kk.y, s);
@@ -947,6 +961,18 @@ __device__ __forceinline__ void attention_layer(const lt_decode_desc& P, const l
         }
         asm volatile("bar.sync 3, 96;" ::: "memory");
     }
+    if (warp >= V_COPIERS_FROM) {
+        for (int g = 4; g < nseg; g++) {
+            v_segment_free_wait(g & 3);
+            const int t0 = g * seg, n = Lc - t0 < seg ? Lc - t0 : seg;
+            for (int e = tid - V_COPIERS_FROM * 32; e < n * HD4; e += DEC_CTHREADS - V_COPIERS_FROM * 32) {
+                const int t = e / HD4, c = e - t * HD4;
+                cp_async16(sV + (size_t)((g & 3) * seg + t) * HD + c * 4, ly->vcache + ((size_t)(t0 + t) * nkv + hk) * HD + c * 4);
+            }
+            cp_async_wait_all();
+            v_segment_full_arrive(g & 3);
+        }
+    }
     if (tid < 64) {
         float m = -1e30f;
         for (int t = tid; t < L; t += 64) m = fmaxf(m, A.sh[t]);
@@ -965,12 +991,33 @@ __device__ __forceinline__ void attention_layer(const lt_decode_desc& P, const l
         pair_sync();
         float Z = warp_tree_sum(__fadd_rn(S->red2[lane], S->red2[lane + 32]));
         Z = __shfl_sync(0xffffffffu, Z, 0);
-        float out = 0.0f;
+        float out = 0.0f, acc = 0.0f;
+        if (in_segments) {
+            for (int g = 0; g < nseg; g++) {
+                if (g >= 4) v_segment_full_wait(g & 3);
+                const int t0 = g * seg, n = Lc - t0 < seg ? Lc - t0 : seg;
+                if (tid < HD) {
+                    const float* vs = sV + (size_t)((g & 3) * seg) * HD + tid;
+                    const float* ps = A.sh + t0;
+                    int t = 0;
+#pragma unroll 2
+                    for (; t + 4 <= n; t += 4) {
+                        const float4 pp = *(const float4*)(ps + t);
+                        const float v0 = vs[t * HD], v1 = vs[(t + 1) * HD], v2 = vs[(t + 2) * HD], v3 = vs[(t + 3) * HD];
+                        acc = __fmaf_rn(pp.x, v0, acc); acc = __fmaf_rn(pp.y, v1, acc);
+                        acc = __fmaf_rn(pp.z, v2, acc); acc = __fmaf_rn(pp.w, v3, acc);
+                    }
+                    for (; t < n; t++) acc = __fmaf_rn(ps[t], vs[t * HD], acc);
+                }
+                if (g + 4 < nseg) v_segment_free_arrive(g & 3);
+            }
+        }
         if (tid < HD) {
-            float acc = 0.0f;
+            if (!in_segments) {
 #pragma unroll 4
-            for (int t = 0; t < vst; t++) acc = __fmaf_rn(A.sh[t], sV[(size_t)t * HD + tid], acc);
-            if (vst < Lc) {
+                for (int t = 0; t < vst; t++) acc = __fmaf_rn(A.sh[t], sV[(size_t)t * HD + tid], acc);
+            }
+            if (!in_segments && vst < Lc) {
                 const float* Vd = ly->vcache + (size_t)hk * HD + tid;
                 const size_t stride = (size_t)nkv * HD;
                 int t = vst;

@@ -318,3 +318,31 @@ def test_generate_from_gguf_equals_engine_on_the_same_weights(tmp_path):
     dr.reset_engine_state()
     got2 = decode_fact.decode(path, prompt, 10)
     assert got2 == want
+
+
+@pytest.mark.parametrize("context", [240, 283, 296, 359, 577, 1003])
+def test_one_kernel_step_in_long_contexts_equals_per_op_graph(context):
+    """Contexts whose cached V rows fill the staging area of an attention CTA, exceed it by a few rows, and pass through it
+    in segments with whole and partial last ones: logits of the one-kernel step and of the per-op graph, bit for bit."""
+    out = []
+    for mode in ("persistent", False):
+        m, w, cfg = _fresh("qwen2.5-0.5b", seed=2, n_layers=2)
+        V = m["cfg"]["vocab"]
+        toks = _prompt(V, context + 8, seed=context)
+        dr._KV_MAX_SEQ = context + 16
+        old = dr._FUSED_STEP
+        dr._FUSED_STEP = mode
+        try:
+            kv = [None] * cfg["n_layers"]
+            gr = dr.GraphRunner(w, cfg, kv)
+            gr.seed(torch.tensor(toks[:context]), torch.arange(context))
+            gr.capture(torch.tensor([toks[context]]), torch.tensor([context]))
+            if mode == "persistent":
+                assert gr.launches_per_token == 1
+            out.append([bits(gr.replay_logits(t).reshape(-1).numpy()).copy() for t in toks[context:]])
+        finally:
+            dr._FUSED_STEP = old
+            dr.apply_production_profile()
+    for i, (a, b) in enumerate(zip(*out)):
+        assert np.array_equal(a, b), i
+    assert dr._lib.device_status() == set()
