@@ -8,7 +8,7 @@
 //   warp 8 : producer, TMA tiles of 64 k (128-byte rows, hardware swizzle) into a ring of shared-memory stages
 //   warp 9 : one thread issues the MMAs; two accumulator sets, so the next tile's MMAs run under this tile's epilogue
 //   warps 0-7 : epilogue
-// fp32 (k_gemm_f32): 64 x 64 tiles on the CUDA cores, every product and sum an fp32 fused multiply-add.
+// fp32 (k_gemm_f32): register-blocked tiles on the CUDA cores, every product and sum an fp32 fused multiply-add.
 #include "lt_dn_common.cuh"
 #include "lt_tc.cuh"
 
@@ -286,62 +286,180 @@ static int launch_tc(const void* W, int ldw, const void* X, int ldx, GemmP P, cu
 
 // ---------------------------------------------------------------------------- fp32
 
-// thread (tx, ty): outputs n = 4 groups of 16 apart, so that a warp's stores are contiguous
-template <bool GLU>
-__global__ void __launch_bounds__(256) k_gemm_f32(const float* __restrict__ W, int ldw, const float* __restrict__ X, int ldx,
-                                                  const __grid_constant__ GemmP P) {
-    __shared__ float sw[GLU ? 2 : 1][16][65], sx[16][65];
-    const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
-    const int n0 = blockIdx.x * 64, t0 = blockIdx.y * 64;
-    float acc[GLU ? 2 : 1][4][4];
+// ---- fp32: every product and sum an fp32 fused multiply-add on the CUDA cores, which bound it.  64 weight rows x 8 MQ
+// tokens per CTA of 128 threads, a thread owns 4 rows (pairs of rows with GLU) x MQ tokens: 4 + MQ 16-byte reads of shared
+// memory per 16 MQ multiply-adds, three stages of 32 k filled by asynchronous copies.  A cluster of S CTAs shares a tile's
+// k, in equal contiguous parts added in rank order through distributed shared memory: a prompt of a few hundred tokens
+// has fewer tiles than the GPU has places for CTAs.  Against 4 x 4 per thread from single floats of one unbuffered stage,
+// no split (M x K x T): 896 x 6656 x 300 703 -> 121 us, 3640 x 896 x 300 109 -> 90, 8192 x 2048 x 512 758 -> 423 (56 % of
+// the multiply-adds' rate), 896 x 6656 x 45 700 -> 51.  Shorter chains of sums: errors equal or smaller.
+constexpr int F32_THREADS = 128, F32_BM = 64, F32_BK = 32, F32_ST = F32_BK + 4, F32_STAGES = 3;
+
+template <bool GLU, int MQ>
+struct F32Cfg {
+    static constexpr int NG = GLU ? 2 : 1, BN = 8 * MQ, ROWS = NG * F32_BM + BN;
+    static constexpr int SMEM = F32_STAGES * ROWS * F32_ST * 4;
+    static_assert(SMEM >= NG * 4 * MQ * F32_THREADS * 4, "the partials fit the stages");
+};
+
+__device__ __forceinline__ void f32_cluster_sync() {
+    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+
+template <bool GLU, int MQ>
+__global__ void __launch_bounds__(F32_THREADS)
+k_gemm_f32(const float* __restrict__ W, int ldw, const float* __restrict__ X, int ldx, int S, const __grid_constant__ GemmP P) {
+    using C = F32Cfg<GLU, MQ>;
+    constexpr int NG = C::NG, BN = C::BN;
+    extern __shared__ __align__(16) float f32_smem[];
+    const int tid = threadIdx.x, n = tid & 15, m = tid >> 4;
+    const int n0 = blockIdx.x * F32_BM, t0 = blockIdx.y * BN, rank = blockIdx.z;
+    const int nk = (P.K + F32_BK - 1) / F32_BK;
+    const int c0 = (int)((long)nk * rank / S), c1 = (int)((long)nk * (rank + 1) / S);
+
+    auto copy = [&](int c, int stage) {
+        float* dst = f32_smem + stage * C::ROWS * F32_ST;
+        if (c < c1) {
 #pragma unroll
-    for (int g = 0; g < (GLU ? 2 : 1); g++)
+            for (int e = tid; e < C::ROWS * (F32_BK / 4); e += F32_THREADS) {
+                const int r = e >> 3, k = c * F32_BK + (e & 7) * 4;          // K is a multiple of 4
+                const float* src;
+                bool ok = k < P.K;
+                if (r < NG * F32_BM) {
+                    const int row = n0 + (r & (F32_BM - 1));
+                    ok = ok && row < P.M;
+                    src = W + (long)((r / F32_BM) * P.up_row + row) * ldw + k;
+                } else {
+                    const int t = t0 + r - NG * F32_BM;
+                    ok = ok && t < P.T;
+                    src = X + (long)t * ldx + k;
+                }
+                asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(smem_u32(dst + r * F32_ST + (e & 7) * 4)),
+                             "l"(ok ? src : W), "r"(ok ? 16 : 0)
+                             : "memory");
+            }
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+
+    float acc[NG][MQ][4];
 #pragma unroll
-        for (int i = 0; i < 4; i++)
+    for (int g = 0; g < NG; g++)
+#pragma unroll
+        for (int i = 0; i < MQ; i++)
 #pragma unroll
             for (int j = 0; j < 4; j++) acc[g][i][j] = 0.0f;
-    const int lr = threadIdx.x >> 2, lk = (threadIdx.x & 3) * 4;     // row and first k this thread loads
-    for (int k0 = 0; k0 < P.K; k0 += 16) {
-        const bool k_ok = k0 + lk < P.K;                             // K is a multiple of 4
 #pragma unroll
-        for (int g = 0; g < (GLU ? 2 : 1); g++) {
-            float4 w = make_float4(0, 0, 0, 0);
-            if (k_ok && n0 + lr < P.M) w = *(const float4*)(W + (long)(g * P.up_row + n0 + lr) * ldw + k0 + lk);
-            sw[g][lk][lr] = w.x; sw[g][lk + 1][lr] = w.y; sw[g][lk + 2][lr] = w.z; sw[g][lk + 3][lr] = w.w;
+    for (int s = 0; s < F32_STAGES - 1; s++) copy(c0 + s, s);
+    int stage = 0;
+    for (int c = c0; c < c1; c++) {
+        asm volatile("cp.async.wait_group %0;" ::"n"(F32_STAGES - 2) : "memory");
+        __syncthreads();                                   // chunk c is there, chunk c - 1 is used up
+        copy(c + F32_STAGES - 1, stage == 0 ? F32_STAGES - 1 : stage - 1);
+        const float4* w4 = (const float4*)(f32_smem + (stage * C::ROWS + n) * F32_ST);
+        const float4* x4 = (const float4*)(f32_smem + (stage * C::ROWS + NG * F32_BM + m * MQ) * F32_ST);
+#pragma unroll 2
+        for (int k = 0; k < F32_BK / 4; k++) {
+            float4 x[MQ];
+#pragma unroll
+            for (int i = 0; i < MQ; i++) x[i] = x4[i * (F32_ST / 4) + k];
+#pragma unroll
+            for (int g = 0; g < NG; g++) {
+                float4 w[4];
+#pragma unroll
+                for (int j = 0; j < 4; j++) w[j] = w4[(g * F32_BM + 16 * j) * (F32_ST / 4) + k];
+#pragma unroll
+                for (int i = 0; i < MQ; i++)
+#pragma unroll
+                    for (int j = 0; j < 4; j++) acc[g][i][j] = fmaf(w[j].x, x[i].x, acc[g][i][j]);
+#pragma unroll
+                for (int i = 0; i < MQ; i++)
+#pragma unroll
+                    for (int j = 0; j < 4; j++) acc[g][i][j] = fmaf(w[j].y, x[i].y, acc[g][i][j]);
+#pragma unroll
+                for (int i = 0; i < MQ; i++)
+#pragma unroll
+                    for (int j = 0; j < 4; j++) acc[g][i][j] = fmaf(w[j].z, x[i].z, acc[g][i][j]);
+#pragma unroll
+                for (int i = 0; i < MQ; i++)
+#pragma unroll
+                    for (int j = 0; j < 4; j++) acc[g][i][j] = fmaf(w[j].w, x[i].w, acc[g][i][j]);
+            }
         }
-        float4 x = make_float4(0, 0, 0, 0);
-        if (k_ok && t0 + lr < P.T) x = *(const float4*)(X + (long)(t0 + lr) * ldx + k0 + lk);
-        sx[lk][lr] = x.x; sx[lk + 1][lr] = x.y; sx[lk + 2][lr] = x.z; sx[lk + 3][lr] = x.w;
+        stage = stage == F32_STAGES - 1 ? 0 : stage + 1;
+    }
+    asm volatile("cp.async.wait_all;" ::: "memory");
+    if (S > 1) {        // partials [g][token][row][thread]; every CTA adds up the tokens of its share
         __syncthreads();
 #pragma unroll
-        for (int k = 0; k < 16; k++) {
-            float b[4];
+        for (int g = 0; g < NG; g++)
 #pragma unroll
-            for (int j = 0; j < 4; j++) b[j] = sx[k][ty + 16 * j];
+            for (int i = 0; i < MQ; i++)
 #pragma unroll
-            for (int g = 0; g < (GLU ? 2 : 1); g++)
+                for (int j = 0; j < 4; j++) f32_smem[((g * MQ + i) * 4 + j) * F32_THREADS + tid] = acc[g][i][j];
+        f32_cluster_sync();
+        const unsigned mine = smem_u32(f32_smem + tid);
 #pragma unroll
-                for (int i = 0; i < 4; i++) {
-                    const float a = sw[g][k][tx + 16 * i];
+        for (int i = 0; i < MQ; i++) {
+            if (i * S / MQ != rank) continue;
 #pragma unroll
-                    for (int j = 0; j < 4; j++) acc[g][i][j] = fmaf(a, b[j], acc[g][i][j]);
+            for (int g = 0; g < NG; g++)
+#pragma unroll
+                for (int j = 0; j < 4; j++) {
+                    float v = 0.0f;
+                    for (int r = 0; r < S; r++) {
+                        unsigned a;
+                        float part;
+                        asm volatile("mapa.shared::cluster.u32 %0, %1, %2;"
+                                     : "=r"(a)
+                                     : "r"(mine + (unsigned)(((g * MQ + i) * 4 + j) * F32_THREADS * 4)), "r"(r));
+                        asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(part) : "r"(a) : "memory");
+                        v = r == 0 ? part : v + part;
+                    }
+                    acc[g][i][j] = v;
                 }
         }
-        __syncthreads();
+        f32_cluster_sync();     // no CTA leaves while another reads its partials
     }
 #pragma unroll
-    for (int i = 0; i < 4; i++) {
-        const int n = n0 + tx + 16 * i;
-        if (n >= P.M) continue;
-        const RowEpi re = row_epi(P.epi, n);
+    for (int j = 0; j < 4; j++) {
+        const int row = n0 + n + 16 * j;
+        if (row >= P.M) continue;
+        const RowEpi re = row_epi(P.epi, row);
 #pragma unroll
-        for (int j = 0; j < 4; j++) {
-            const int t = t0 + ty + 16 * j;
-            if (t >= P.T) continue;
-            if (GLU) glu_store<float>(P.epi, P.Y, (long)t * P.ldy + n, acc[0][i][j], acc[GLU ? 1 : 0][i][j]);
-            else epi_store<float>(P.epi, re, P.Y, t, P.ldy, n, acc[0][i][j]);
+        for (int i = 0; i < MQ; i++) {
+            const int t = t0 + m * MQ + i;
+            if (t >= P.T || i * S / MQ != rank) continue;
+            if (GLU) glu_store<float>(P.epi, P.Y, (long)t * P.ldy + row, acc[0][i][j], acc[NG - 1][i][j]);
+            else epi_store<float>(P.epi, re, P.Y, t, P.ldy, row, acc[0][i][j]);
         }
     }
+}
+
+template <bool GLU, int MQ>
+static int launch_f32(const void* W, int ldw, const void* X, int ldx, const GemmP& P, cudaStream_t s) {
+    using C = F32Cfg<GLU, MQ>;
+    static PerDeviceOnce once;
+    if (once.first()) LT_CUDA(cudaFuncSetAttribute(k_gemm_f32<GLU, MQ>, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM));
+    const long gx = (P.M + F32_BM - 1) / F32_BM, gy = (P.T + C::BN - 1) / C::BN;
+    LT_REQUIRE(gy <= 65535, "lt_dn_linear: T=%d too large", P.T);
+    // parts of k: until three CTAs per SM are there, each with at least eight chunks
+    int S = 1;
+    while (S < 4 && gx * gy * S < 3 * sm_count() && P.K / F32_BK / (2 * S) >= 8) S *= 2;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)gx, (unsigned)gy, (unsigned)S);
+    cfg.blockDim = dim3(F32_THREADS);
+    cfg.dynamicSmemBytes = C::SMEM;
+    cfg.stream = s;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = at[0].val.clusterDim.y = 1;
+    at[0].val.clusterDim.z = (unsigned)S;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    return check_launch("lt_dn_linear", 1,
+                        cudaLaunchKernelEx(&cfg, k_gemm_f32<GLU, MQ>, (const float*)W, ldw, (const float*)X, ldx, S, P));
 }
 
 // tile width: fewest (waves x time of a tile); a tile costs its columns plus what does not shrink with them
@@ -386,11 +504,10 @@ extern "C" int lt_dn_linear(const void* W, int ldw, const void* X, int ldx, void
     P.Y = Y; P.M = M; P.K = K; P.T = T; P.ldy = ldy; P.epi = *h_epi; P.up_row = M;
     const bool glu = h_epi->kind == LT_DN_GLU;
     if (f32) {
-        dim3 grid((M + 63) / 64, (T + 63) / 64);
-        LT_REQUIRE(grid.y <= 65535, "lt_dn_linear: T=%d too large", T);
-        if (glu) k_gemm_f32<true><<<grid, 256, 0, s>>>((const float*)W, ldw, (const float*)X, ldx, P);
-        else k_gemm_f32<false><<<grid, 256, 0, s>>>((const float*)W, ldw, (const float*)X, ldx, P);
-        return check_launch("lt_dn_linear");
+        // 64 tokens per CTA while that gives every SM a tile, else 32 (half the reuse, twice the CTAs)
+        const bool wide = (long)((M + 63) / 64) * ((T + 63) / 64) >= sm_count();
+        if (glu) return wide ? launch_f32<true, 8>(W, ldw, X, ldx, P, s) : launch_f32<true, 4>(W, ldw, X, ldx, P, s);
+        return wide ? launch_f32<false, 8>(W, ldw, X, ldx, P, s) : launch_f32<false, 4>(W, ldw, X, ldx, P, s);
     }
     const int nt = variant ? variant : choose_nt(M, T, glu);
     if (glu) {

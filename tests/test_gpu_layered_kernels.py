@@ -371,3 +371,26 @@ def test_window_edge_shows(f32, T):
         sees = 0 <= t - star < W
         assert abs(o[t, 3] - (4.0 if sees else 0.0)) < 0.05, (t, o[t, 3])
         assert abs(o[t, 16 + 7] - (0.0 if sees else 4.0)) < 0.05, (t, o[t, 23])
+
+
+@pytest.mark.parametrize("M,K,T", [(70, 1096, 33), (65, 520, 1), (896, 2080, 31), (4800, 544, 130)])
+def test_fp32_linear_with_parts_of_k(M, K, T):
+    """Few tiles of long rows: a cluster shares k (four and two parts, with a ragged last chunk, rows and tokens), every
+    epilogue; and enough tiles for the wide form.  Bound: 4 roundings' growth of a K-term fp32 sum of O(1) products."""
+    W, X = _t((2 * M, K), 8, 1, K ** -0.5), _t((T, K), 9, 1)
+    tol = 2e-6 * K ** 0.5
+    v = _np(X) @ _np(W).T
+    Y = torch.full((T, M + 4), 7.0, device="cuda")
+    e = P.epilogue(segs=[(M // 3, "silu", 1.0), (M, None, 0.5)])
+    _lib.call("lt_dn_linear", W.data_ptr(), K, X.data_ptr(), K, Y.data_ptr(), M + 4, 1, M, K, T, ctypes.byref(e), 0, stream())
+    _close(_np(Y)[:, :M], np.concatenate([L.silu(v[:, :M // 3]), 0.5 * v[:, M // 3:M]], axis=1), tol)
+    assert (_np(Y)[:, M:] == 7.0).all()
+    ls, R = torch.randn(M).cuda(), torch.randn(T, M).cuda()
+    r0 = _np(R)
+    e = P.epilogue(_lib.DN_RESID, ls=ls)
+    _lib.call("lt_dn_linear", W.data_ptr(), K, X.data_ptr(), K, R.data_ptr(), M, 1, M, K, T, ctypes.byref(e), 0, stream())
+    _close(_np(R), r0 + v[:, :M] * _np(ls), 3 * tol)
+    Z = torch.empty(T, M, device="cuda")
+    e = P.epilogue(_lib.DN_GLU, out_f32=True)
+    _lib.call("lt_dn_linear", W.data_ptr(), K, X.data_ptr(), K, Z.data_ptr(), M, 1, M, K, T, ctypes.byref(e), 0, stream())
+    _close(_np(Z), L.gelu_tanh(v[:, :M]) * v[:, M:], 6 * tol)
