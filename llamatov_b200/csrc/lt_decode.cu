@@ -110,6 +110,18 @@ __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wai
 
 __device__ __forceinline__ void consumer_sync() { asm volatile("bar.sync 1, %0;" ::"n"(DEC_CTHREADS) : "memory"); }
 __device__ __forceinline__ void pair_sync() { asm volatile("bar.sync 2, 64;" ::: "memory"); }   // warps 0 and 1
+// 32 bytes of global memory, from L2
+__device__ __forceinline__ void ld_sector(const float* p, float (&v)[8], bool aligned) {
+    if (aligned) {
+        asm volatile("ld.global.L1::no_allocate.v8.f32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+                     : "=f"(v[0]), "=f"(v[1]), "=f"(v[2]), "=f"(v[3]), "=f"(v[4]), "=f"(v[5]), "=f"(v[6]), "=f"(v[7])
+                     : "l"(p)
+                     : "memory");
+    } else {
+        const float4 a = __ldcg((const float4*)p), b = __ldcg((const float4*)p + 1);
+        v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w; v[4] = b.x; v[5] = b.y; v[6] = b.z; v[7] = b.w;
+    }
+}
 // Segments of cached V rows (attention CTA): buffer b of four is full / free.  Warps 0 and 1 fold, warps V_COPIERS_FROM.. copy.
 constexpr int V_COPIERS_FROM = 3;
 constexpr int V_PARTIES = 64 + DEC_CTHREADS - V_COPIERS_FROM * 32;
@@ -825,7 +837,7 @@ __device__ __forceinline__ void attention_layer(const lt_decode_desc& P, const l
     // Cached V rows are staged in shared memory.  A context with more rows than fit goes through it in segments of seg
     // rows, four buffers: the first four now, the others during the V fold, each when the one four before it is folded
     // (warps 3.. copy, warps 0 and 1 fold).  Folding the rest from global memory, eight rows per round trip to L2, cost
-    // more than the whole rest of the layer: 1000 positions 1178 us per token, now 811 us (32 positions: 376).
+    // more than the whole rest of the layer: 1000 positions 1178 us per token, now 811 us (32 positions: 380).
     const int seg = vcap / 16 * 4;
     const bool in_segments = Lc > vcap && seg > 0;
     const int nseg = in_segments ? (Lc + seg - 1) / seg : 0;
@@ -932,16 +944,37 @@ __device__ __forceinline__ void attention_layer(const lt_decode_desc& P, const l
         }
         if (hf == 1 && t < L) A.sh[t] = __fmul_rn(s, P.scale);
     }
-    for (int t = tid + KPOS; t < L; t += DEC_CTHREADS) {     // contexts longer than the registers hold
-        const float4* k4 = (room && t == pos) ? (const float4*)A.kn
-                                              : (const float4*)(ly->kcache + ((size_t)t * nkv + hk) * HD);
+    // contexts longer than the registers hold: a thread per position, half a row on its way at once, by whole sectors
+    // (16-byte loads of 32 different rows fetch every sector twice: the carve-out leaves no L1 to keep the other half).  1000 positions: 811 -> 708 us per token
+    for (int t = tid + KPOS; t < L; t += DEC_CTHREADS) {
         const float4* q4 = (const float4*)A.q;
         float s = 0.0f;
-#pragma unroll 8
-        for (int i = 0; i < HD4; i++) {
-            const float4 qq = q4[i], kk = k4[i];
-            s = __fmaf_rn(qq.x, kk.x, s); s = __fmaf_rn(qq.y, kk.y, s);
-            s = __fmaf_rn(qq.z, kk.z, s); s = __fmaf_rn(qq.w, kk.w, s);
+        if (room && t == pos) {
+            const float4* k4 = (const float4*)A.kn;
+#pragma unroll 1
+            for (int i = 0; i < HD4; i++) {
+                const float4 qq = q4[i], kk = k4[i];
+                s = __fmaf_rn(qq.x, kk.x, s); s = __fmaf_rn(qq.y, kk.y, s);
+                s = __fmaf_rn(qq.z, kk.z, s); s = __fmaf_rn(qq.w, kk.w, s);
+            }
+        } else {
+            const float* kp = ly->kcache + ((size_t)t * nkv + hk) * HD;
+            const bool sectors = (reinterpret_cast<uintptr_t>(kp) & 31u) == 0;
+            constexpr int HALF_LOADS = HD / 16;      // 32-byte loads of half a row
+#pragma unroll 1
+            for (int half = 0; half < 2; half++) {
+                float kk[HALF_LOADS][8];
+#pragma unroll
+                for (int i = 0; i < HALF_LOADS; i++) ld_sector(kp + (half * HALF_LOADS + i) * 8, kk[i], sectors);
+#pragma unroll
+                for (int i = 0; i < HALF_LOADS; i++) {
+                    const float4 qa = q4[(half * HALF_LOADS + i) * 2], qb = q4[(half * HALF_LOADS + i) * 2 + 1];
+                    s = __fmaf_rn(qa.x, kk[i][0], s); s = __fmaf_rn(qa.y, kk[i][1], s);
+                    s = __fmaf_rn(qa.z, kk[i][2], s); s = __fmaf_rn(qa.w, kk[i][3], s);
+                    s = __fmaf_rn(qb.x, kk[i][4], s); s = __fmaf_rn(qb.y, kk[i][5], s);
+                    s = __fmaf_rn(qb.z, kk[i][6], s); s = __fmaf_rn(qb.w, kk[i][7], s);
+                }
+            }
         }
         A.sh[t] = __fmul_rn(s, P.scale);
     }
