@@ -24,6 +24,10 @@
 //               into a ring of shared-memory stages; a stage = one chunk of CB blocks
 //   warp EW+1 : one thread issues the CB MMAs of a stage into a ring of TMEM slots and commits
 //   warps 0..EW-1 : epilogue, TMEM -> registers -> fp32 fold -> Y
+// Split rows of blocks (S > 1): a cluster of S CTAs shares a tile, CTA r visits the groups g = r mod S, a whole subtree of
+// the tree; the levels across those subtrees and inside a group are added by the CTA that finishes a column, from all
+// CTAs' partials in its shared memory.  Small batches need it: a matrix of 4096 rows has 32 row tiles for 148 SMs
+// (4096 x 14336, 24 columns: 64 CTAs 57 us, 128 CTAs 37 us; 9 columns: 32 CTAs 67 us, 128 CTAs 31 us).
 // Every wait is bounded: after the limit a CTA sets LT_STATUS_WAIT_TIMEOUT, all its later waits
 // return at once, it drains and frees its tensor memory.
 #include "lt_tc.cuh"
@@ -55,6 +59,48 @@ __device__ __forceinline__ void tmem_ld_wait(int (&v)[CB][CW]) {
         for (int c = 0; c < CW; c += 4) reg_fence4(&v[i][c]);
 }
 
+// ---- cluster
+__device__ __forceinline__ unsigned cluster_rank() {
+    unsigned r;
+    asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+    return r;
+}
+__device__ __forceinline__ unsigned map_rank(unsigned addr, unsigned rank) {   // the same shared address in another CTA of the cluster
+    unsigned r;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(addr), "r"(rank));
+    return r;
+}
+__device__ __forceinline__ void cluster_sync() {
+    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+__device__ __forceinline__ void arrive_remote(unsigned bar) {
+    asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(bar) : "memory");
+}
+__device__ __forceinline__ bool try_wait_cluster(unsigned long long* bar, unsigned parity) {
+    unsigned ok;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}"
+        : "=r"(ok)
+        : "r"(smem_u32(bar)), "r"(parity)
+        : "memory");
+    return ok != 0;
+}
+__device__ __forceinline__ void wait_cluster(unsigned long long* bar, unsigned parity, volatile int* abort_flag, int* status) {
+    if (try_wait_cluster(bar, parity)) return;
+    const long long t0 = clock64();
+    while (!try_wait_cluster(bar, parity)) {
+        if (*abort_flag) return;
+        if (clock64() - t0 > WAIT_LIMIT) {
+            *abort_flag = 1;
+            atomicOr(status, LT_STATUS_WAIT_TIMEOUT);
+            return;
+        }
+    }
+}
+
 constexpr int ilog2(int v) { return v <= 1 ? 0 : 1 + ilog2(v >> 1); }
 
 struct Params {
@@ -65,26 +111,30 @@ struct Params {
     int* status;
     int M, K, T;
     int row_tiles, t_tiles;
+    int nstage;     // stages of the ring, even, at most 8
     int resid_ld;   // 0: Resid[n] for every column (bias); else Resid[t * resid_ld + n]
 };
 
-template <int NT, int CB, int EW>
+template <int NT, int CB, int EW, int S>
 struct Cfg {
     static constexpr int CW = NT * 4 / EW;             // columns per epilogue thread
-    static constexpr int G = 32 / CB;                  // lane groups
+    static constexpr int G = 32 / CB / S;              // lane groups that a CTA of the cluster visits
     static constexpr int LV = ilog2(G);                // stack depth
+    static constexpr int QPR = NT / 4 / S;             // quads of columns that a CTA finishes
+    static constexpr int XCHG = S > 1 ? S * QPR * CB * TM * 16 : 0;   // bytes of the partials of those columns
     static constexpr int MW = 2;                       // MMA-issuing warps
     static constexpr int THREADS = (EW + 1 + MW) * 32;
     static constexpr int W_STAGE = CB * TM * 32;       // bytes: one stage = one chunk of CB blocks
     static constexpr int X_STAGE = CB * NT * 32;
     static constexpr int STAGE = W_STAGE + ((X_STAGE + 1023) / 1024) * 1024;
-    static constexpr int NSTAGE = CB == 4 ? 4 : (CB == 2 ? 6 : 8);
+    static constexpr int NSTAGE_MIN = CB == 4 ? 4 : (CB == 2 ? 6 : 8);
     static constexpr int SLOT_COLS = CB * NT;
     static constexpr int NSLOT = TMEM_COLS / SLOT_COLS;
     static constexpr int LB = CB * CW <= 16 ? CB : (CB >= 2 && CW <= 8 ? 2 : 1);   // blocks per TMEM round trip
     static_assert(EW % 4 == 0 && (CW == 4 || CW == 8 || CW == 16), "epilogue shape");
     static_assert(NSLOT >= 2 && NSLOT <= 16 && (NSLOT & (NSLOT - 1)) == 0, "TMEM slots");
     static_assert(W_STAGE % 1024 == 0, "stages keep 1024-byte alignment");
+    static_assert(S == 1 || (EW == 8 && CW == 8 && NT == 16 && (S == 2 || S == 4)), "the exchange deals quads to ranks");
 };
 
 struct Barriers {
@@ -92,23 +142,36 @@ struct Barriers {
     unsigned long long tfull[16], tempty[16];
     unsigned tmem_base;
     int abort_flag;
+    unsigned long long xfull, xfree[4];   // all partials of this CTA's columns are here; rank r has read what it was sent
     int next_start[32];   // per visiting position: first block of the next group that has blocks, -1 = none
 };
 
-template <int NT, int CB, int EW>
-__global__ void __launch_bounds__(Cfg<NT, CB, EW>::THREADS, 1)
+template <int NT, int CB, int EW, int S>
+__global__ void __launch_bounds__(Cfg<NT, CB, EW, S>::THREADS, 1)
 k_q8_gemm_tc(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUtensorMap tmX, const Params P) {
-    using C = Cfg<NT, CB, EW>;
-    constexpr int CW = C::CW, G = C::G, LV = C::LV, NSLOT = C::NSLOT, NSTAGE = C::NSTAGE, LB = C::LB, MW = C::MW;
+    using C = Cfg<NT, CB, EW, S>;
+    constexpr int CW = C::CW, G = C::G, LV = C::LV, NSLOT = C::NSLOT, LB = C::LB, MW = C::MW;
     extern __shared__ __align__(1024) unsigned char smem_raw[];
     // 1024-byte aligned carve-up: stages (weights, then activations), barriers, activation scales
     unsigned char* base = (unsigned char*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
-    Barriers* B = (Barriers*)(base + NSTAGE * C::STAGE);
-    float* xs = (float*)((unsigned char*)B + 1024);
+    Barriers* B = (Barriers*)(base + P.nstage * C::STAGE);
+    float* xchg = (float*)((unsigned char*)B + 1024);
+    float* xs = (float*)((unsigned char*)xchg + C::XCHG);
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int nb = P.K >> 5;
+    const int nb = P.K >> 5, NSTAGE = P.nstage;
     const int tiles = P.row_tiles * P.t_tiles;
+    const int rank = S > 1 ? (int)cluster_rank() : 0;
+    const int tile_first = blockIdx.x / S, tile_step = gridDim.x / S;
+    auto group = [&](int gi) {   // the gi-th group this CTA visits
+        return rank + S * (LV > 0 ? (int)(__brev((unsigned)gi) >> (32 - (LV > 0 ? LV : 1))) : 0);
+    };
+    unsigned chunks = 0;         // of a tile, in this CTA
+#pragma unroll
+    for (int gi = 0; gi < G; gi++) {
+        const int b0 = CB * group(gi);
+        chunks += b0 < nb ? (unsigned)((nb - b0 + 31) >> 5) : 0u;
+    }
     volatile int* abort_flag = &B->abort_flag;
 
     if (tid == 0) {
@@ -120,11 +183,13 @@ k_q8_gemm_tc(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CU
             mbar_init(&B->tfull[s], 1);
             mbar_init(&B->tempty[s], EW);
         }
+        mbar_init(&B->xfull, 4 * S);
+        for (int s = 0; s < 4; s++) mbar_init(&B->xfree[s], EW);
         B->abort_flag = 0;
         for (int gi = 0; gi < G; gi++) {
             int nxt = -1;
             for (int gj = gi + 1; gj < G && nxt < 0; gj++) {
-                const int b0 = CB * (int)(__brev((unsigned)gj) >> (32 - LV));
+                const int b0 = CB * group(gj);
                 if (b0 < nb) nxt = b0;
             }
             B->next_start[gi] = nxt;
@@ -139,7 +204,9 @@ k_q8_gemm_tc(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CU
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
     tc_fence_before();
-    __syncthreads();
+    __syncwarp();
+    if (S > 1) cluster_sync();   // the other CTAs' barriers are initialised
+    else __syncthreads();
     tc_fence_after();
     const unsigned tmem = B->tmem_base;
 
@@ -147,19 +214,23 @@ k_q8_gemm_tc(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CU
     if (warp == EW) {
         // ------------------------------------------------------------------ producer
         if (lane == 0) {
-            unsigned it = 0;   // chunks issued
-            for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
+            int s = 0;             // stage of the next chunk
+            unsigned phase = 0;    // of its barriers
+            for (int tile = tile_first; tile < tiles; tile += tile_step) {
                 const int rt = tile / P.t_tiles, tt = tile - rt * P.t_tiles;
                 const int row0 = rt * TM, t0 = tt * NT;
                 for (int gi = 0; gi < G; gi++) {
-                    const int g = (int)(__brev((unsigned)gi) >> (32 - LV));
-                    for (int b0 = CB * g; b0 < nb; b0 += 32, it++) {
-                        const int s = it % NSTAGE;
+                    const int g = group(gi);
+                    for (int b0 = CB * g; b0 < nb; b0 += 32) {
                         unsigned char* st = base + s * C::STAGE;
-                        mbar_wait<64>(&B->empty[s], ((it / NSTAGE) & 1) ^ 1, abort_flag, P.status);
+                        mbar_wait<64>(&B->empty[s], phase ^ 1, abort_flag, P.status);
                         mbar_expect_tx(&B->full[s], C::W_STAGE + C::X_STAGE);
                         tma_load_2d(st, &tmW, b0 * 32, row0, &B->full[s]);
                         tma_load_2d(st + C::W_STAGE, &tmX, b0 * 32, t0, &B->full[s]);
+                        if (++s == NSTAGE) {
+                            s = 0;
+                            phase ^= 1;
+                        }
                     }
                 }
             }
@@ -174,13 +245,13 @@ k_q8_gemm_tc(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CU
                                        ((unsigned)(TM >> 4) << 24);
             const unsigned long long wdesc0 = smem_desc<CB>(smem_u32(base));
             const unsigned long long xdesc0 = smem_desc<CB>(smem_u32(base) + C::W_STAGE);
-            const unsigned chunks = (unsigned)(nb / CB);
             int my_tiles = 0;
-            for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x) my_tiles++;
+            for (int tile = tile_first; tile < tiles; tile += tile_step) my_tiles++;
             const unsigned total = (unsigned)my_tiles * chunks;
-            for (unsigned it = (unsigned)(warp - (EW + 1)); it < total; it += MW) {
-                const unsigned s = it % NSTAGE, slot = it % NSLOT;
-                mbar_wait<32>(&B->full[s], (it / NSTAGE) & 1, abort_flag, P.status);
+            unsigned s = (unsigned)(warp - (EW + 1)), phase = 0;     // stage of chunk it, phase of its barriers
+            for (unsigned it = s; it < total; it += MW) {
+                const unsigned slot = it % NSLOT;
+                mbar_wait<32>(&B->full[s], phase, abort_flag, P.status);
                 mbar_wait<32>(&B->tempty[slot], ((it / NSLOT) & 1) ^ 1, abort_flag, P.status);
                 tc_fence_after();
                 // descriptors differ from the first stage's only in the start address (16-byte units)
@@ -192,6 +263,11 @@ k_q8_gemm_tc(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CU
                     mma_i8(d0 + i * NT, wd0 + 2 * i, xd0 + 2 * i, idesc);
                 mma_commit(&B->empty[s]);     // the stage may be refilled once these MMAs have read it
                 mma_commit(&B->tfull[slot]);  // and the slot holds the block sums
+                s += MW;
+                if (s >= (unsigned)NSTAGE) {
+                    s -= (unsigned)NSTAGE;
+                    phase ^= 1;
+                }
             }
         }
     } else {
@@ -202,9 +278,10 @@ k_q8_gemm_tc(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CU
         const int col0 = cg * CW;
         const unsigned lane_addr = ((unsigned)(q * 32) << 16) + (unsigned)col0;
         int my_tiles = 0;
-        for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x) my_tiles++;
-        const unsigned total = (unsigned)my_tiles * (unsigned)(nb / CB);   // chunks this thread consumes
+        for (int tile = tile_first; tile < tiles; tile += tile_step) my_tiles++;
+        const unsigned total = (unsigned)my_tiles * chunks;                // chunks this thread consumes
         unsigned it = 0;                                                   // chunks consumed so far
+        unsigned turn = 0;                                                 // tiles exchanged so far
         auto scale_row = [&](int tile) {   // this thread's row of weight scales in a tile (row 0 if out of range)
             int r = (tile / P.t_tiles) * TM + q * 32 + lane;
             if (r >= P.M) r = 0;
@@ -218,21 +295,22 @@ k_q8_gemm_tc(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CU
             return w;
         };
         uint2 wnext = make_uint2(0u, 0u);
-        if (total > 0) wnext = scales_at(scale_row(blockIdx.x));
+        if (total > 0) wnext = scales_at(scale_row(tile_first) + CB * rank);
 
-        for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
+        for (int tile = tile_first; tile < tiles; tile += tile_step) {
             const int rt = tile / P.t_tiles, tt = tile - rt * P.t_tiles;
             const int row = rt * TM + q * 32 + lane, t0 = tt * NT;
             const bool row_ok = row < P.M;
             const __half* wdrow = scale_row(tile);
-            const __half* wdrow_next = scale_row(tile + gridDim.x < tiles ? tile + (int)gridDim.x : tile);
+            const __half* wdrow_next = scale_row(tile + tile_step < tiles ? tile + tile_step : tile) + CB * rank;
 
             // activation scales of this column tile: xs[b][c] = f32(Xd[t0 + c, b])
             asm volatile("bar.sync 1, %0;" ::"n"(EW * 32) : "memory");
             for (int c = warp; c < NT; c += EW) {
                 const bool ok = t0 + c < P.T;
                 const __half* xr = P.Xd + (long)(ok ? t0 + c : 0) * nb;
-                for (int b = lane; b < nb; b += 32) xs[b * NT + c] = ok ? __half2float(xr[b]) : 0.0f;
+                for (int b = lane; b < nb; b += 32)
+                    if (S == 1 || ((b / CB) & (S - 1)) == rank) xs[b * NT + c] = ok ? __half2float(xr[b]) : 0.0f;
             }
             asm volatile("bar.sync 1, %0;" ::"n"(EW * 32) : "memory");
 
@@ -240,7 +318,7 @@ k_q8_gemm_tc(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CU
             float fin[CB][CW];
 #pragma unroll
             for (int gi = 0; gi < G; gi++) {
-                const int g = (int)(__brev((unsigned)gi) >> (32 - LV));
+                const int g = group(gi);
                 float leaf[CB][CW];
 #pragma unroll
                 for (int i = 0; i < CB; i++)
@@ -321,6 +399,67 @@ k_q8_gemm_tc(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CU
                     }
                 }
             }
+            if (S > 1) {
+                // this thread's CB x CW partials go to the CTAs that finish the columns, by quads:
+                // [source rank][quad of the rank][lane of the group][row][4]
+                constexpr int QPR = C::QPR;
+                const int r = q * 32 + lane;
+#pragma unroll
+                for (int h = 0; h < CW / 4; h++) {
+                    const unsigned quad = (unsigned)(cg * (CW / 4) + h), dst = quad / QPR;
+                    wait_cluster(&B->xfree[dst], (turn & 1) ^ 1, abort_flag, P.status);
+                    const unsigned buf = map_rank(smem_u32(xchg), dst) + ((unsigned)rank * QPR + quad % QPR) * (CB * TM * 16);
+#pragma unroll
+                    for (int i = 0; i < CB; i++)
+                        asm volatile("st.shared::cluster.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(buf + (unsigned)((i * TM + r) * 16)),
+                                     "f"(fin[i][4 * h]), "f"(fin[i][4 * h + 1]), "f"(fin[i][4 * h + 2]), "f"(fin[i][4 * h + 3])
+                                     : "memory");
+                    // one arrival per warp and destination (both quads of a warp may have the same)
+                    if (QPR == 1 || h == CW / 4 - 1) {
+                        __syncwarp();
+                        if (lane == 0) arrive_remote(map_rank(smem_u32(&B->xfull), dst));
+                    }
+                }
+                wait_cluster(&B->xfull, turn & 1, abort_flag, P.status);
+                // columns 4 * QPR * rank + cg * NC ..: levels across the ranks, then across the lanes of a group
+                constexpr int NC = 2 * QPR;
+                float y[NC];
+#pragma unroll
+                for (int c = 0; c < NC; c++) {
+                    const int col = cg * NC + c;      // among this rank's columns
+                    float part[CB];
+#pragma unroll
+                    for (int i = 0; i < CB; i++) {
+                        float pr[S];
+#pragma unroll
+                        for (int k = 0; k < S; k++) pr[k] = xchg[(((k * QPR + col / 4) * CB + i) * TM + r) * 4 + col % 4];
+#pragma unroll
+                        for (int s = S / 2; s >= 1; s >>= 1)
+#pragma unroll
+                            for (int k = 0; k < s; k++) pr[k] = __fadd_rn(pr[k], pr[k + s]);
+                        part[i] = pr[0];
+                    }
+#pragma unroll
+                    for (int s = CB / 2; s >= 1; s >>= 1)
+#pragma unroll
+                        for (int i = 0; i < s; i++) part[i] = __fadd_rn(part[i], part[i + s]);
+                    y[c] = part[0];
+                }
+                __syncwarp();
+                if (lane < S) arrive_remote(map_rank(smem_u32(&B->xfree[rank]), (unsigned)lane));
+                turn++;
+                if (row_ok) {
+#pragma unroll
+                    for (int c = 0; c < NC; c++) {
+                        const int t = t0 + 4 * QPR * rank + cg * NC + c;
+                        if (t < P.T) {
+                            if (P.Resid != nullptr) y[c] = __fadd_rn(y[c], P.Resid[(long)t * P.resid_ld + row]);
+                            P.Y[(long)t * P.M + row] = y[c];
+                        }
+                    }
+                }
+                continue;
+            }
             // last levels of the tree across the CB lanes of a group: strides CB/2, ..., 1
 #pragma unroll
             for (int s = CB / 2; s >= 1; s >>= 1)
@@ -352,7 +491,9 @@ k_q8_gemm_tc(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CU
         while (clock64() - t0 < 2000000LL) {
         }
     }
-    __syncthreads();
+    __syncwarp();
+    if (S > 1) cluster_sync();   // no CTA leaves while another may still write to its shared memory
+    else __syncthreads();
     if (warp == EW + 1) {
         tc_fence_after();
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"((unsigned)TMEM_COLS)
@@ -386,36 +527,78 @@ static int make_map(CUtensorMap* m, const void* ptr, int rows, int K, int box_k,
     return LT_OK;
 }
 
-template <int NT, int CB, int EW>
+static int sm_count() {
+    int dev = 0, sms = 148;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    return sms < 4 ? 4 : sms;
+}
+
+template <int NT, int CB, int EW, int S>
 static int launch(const int8_t* Wq, const uint16_t* Wd, const int8_t* Xq, const uint16_t* Xd, const float* Resid,
                   int resid_ld, float* Y, int M, int K, int T, cudaStream_t s) {
-    using C = Cfg<NT, CB, EW>;
+    using C = Cfg<NT, CB, EW, S>;
     const int nb = K / 32;
     CUtensorMap tmW, tmX;
     int rc = make_map(&tmW, Wq, M, K, CB * 32, TM);
     if (rc != LT_OK) return rc;
     rc = make_map(&tmX, Xq, T, K, CB * 32, NT);
     if (rc != LT_OK) return rc;
-    const size_t smem = 1024 + (size_t)C::NSTAGE * C::STAGE + 1024 + (size_t)nb * NT * 4;
+    // as many stages as fit: a chunk of 18 KB is on its way for a microsecond or two (4 stages -> 8: 28672 x 4096 x 512
+    // 727 -> 684 us, 128256 x 4096 x 32 210 -> 204, narrow batches within 3 % either way)
+    const size_t rest = 1024 + 1024 + C::XCHG + (size_t)nb * NT * 4;
+    int nstage = C::NSTAGE_MIN;
+    while (nstage < 8 && rest + (size_t)(nstage + 2) * C::STAGE <= 220 * 1024) nstage += 2;
+    const size_t smem = rest + (size_t)nstage * C::STAGE;
     LT_REQUIRE(smem <= 220 * 1024, "lt_q8_gemm_tc: K=%d needs %zu bytes of shared memory per CTA", K, smem);
     static PerDeviceOnce attr_once;
     if (attr_once.first()) {
-        LT_CUDA(cudaFuncSetAttribute(k_q8_gemm_tc<NT, CB, EW>, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024));
+        LT_CUDA(cudaFuncSetAttribute(k_q8_gemm_tc<NT, CB, EW, S>, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024));
     }
     Params P;
     P.Wd = (const __half*)Wd; P.Xd = (const __half*)Xd; P.Resid = Resid; P.Y = Y;
     P.status = device_status_ptr();
     LT_REQUIRE(P.status != nullptr, "lt_q8_gemm_tc: status word unavailable");
-    P.M = M; P.K = K; P.T = T; P.resid_ld = resid_ld;
+    P.M = M; P.K = K; P.T = T; P.resid_ld = resid_ld; P.nstage = nstage;
     P.row_tiles = (M + TM - 1) / TM;
     P.t_tiles = (T + NT - 1) / NT;
-    int dev = 0, sms = 148;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     const long tiles = (long)P.row_tiles * P.t_tiles;
-    const int grid = (int)(tiles < sms ? tiles : sms);
-    k_q8_gemm_tc<NT, CB, EW><<<grid, C::THREADS, smem, s>>>(tmW, tmX, P);
-    return check_launch("lt_q8_gemm_tc");
+    const int room = sm_count() / S;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)((tiles < room ? tiles : room) * S));
+    cfg.blockDim = dim3(C::THREADS);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = s;
+    cudaLaunchAttribute at[1];
+    if (S > 1) {
+        at[0].id = cudaLaunchAttributeClusterDimension;
+        at[0].val.clusterDim.x = S;
+        at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+        cfg.attrs = at;
+        cfg.numAttrs = 1;
+    }
+    return check_launch("lt_q8_gemm_tc", 1, cudaLaunchKernelEx(&cfg, k_q8_gemm_tc<NT, CB, EW, S>, tmW, tmX, P));
+}
+
+// How many CTAs share a 16-column tile: the split whose busiest CTA has least to do.  A tile costs a CTA its chunks and
+// a fixed part, larger with the exchange (in chunks of about half a microsecond, from 4096 x 4096 and 4096 x 14336 at 16
+// and 32 columns).  Clusters of four get a place only where a GPC has four SMs free: 32 of them are counted on.
+static int choose_split(int M, int K, int T) {
+    const int sms = sm_count(), nb = K / 32;
+    const long tiles = (long)((M + TM - 1) / TM) * ((T + 15) / 16);
+    if ((size_t)1024 + Cfg<16, 4, 8, 2>::NSTAGE_MIN * Cfg<16, 4, 8, 2>::STAGE + 1024 + Cfg<16, 4, 8, 2>::XCHG + (size_t)nb * 64 > 220 * 1024) return 1;
+    int best = 1;
+    double best_cost = 0.0;
+    for (int S = 1; S <= 4; S *= 2) {
+        const long room = S == 4 ? sms * 32 / 148 : sms / S;
+        const long rounds = (tiles + room - 1) / room;
+        const double cost = (double)rounds * ((double)((nb / 4 + S - 1) / S) + (S == 1 ? 1.5 : 4.0));
+        if (S == 1 || cost < best_cost) {
+            best = S;
+            best_cost = cost;
+        }
+    }
+    return best;
 }
 
 }  // namespace tc
@@ -434,10 +617,15 @@ extern "C" int lt_q8_gemm_tc(const int8_t* Wq, const uint16_t* Wd, const int8_t*
     LT_REQUIRE(Resid == nullptr || resid_ld != 0 || T == 1 || (const void*)Y != (const void*)Resid,
                "lt_q8_gemm_tc: Y may alias Resid only when Resid has one row per column");
     cudaStream_t s = (cudaStream_t)stream;
-    if (variant == 0) variant = 1;
-    if (variant == 1) return tc::launch<16, 4, 8>(Wq, Wd, Xq, Xd, Resid, resid_ld, Y, M, K, T, s);
-    if (variant == 2) return tc::launch<32, 1, 8>(Wq, Wd, Xq, Xd, Resid, resid_ld, Y, M, K, T, s);
-    if (variant == 3) return tc::launch<16, 4, 16>(Wq, Wd, Xq, Xd, Resid, resid_ld, Y, M, K, T, s);
+    if (variant == 0) {
+        const int S = tc::choose_split(M, K, T);
+        if (S == 4) return tc::launch<16, 4, 8, 4>(Wq, Wd, Xq, Xd, Resid, resid_ld, Y, M, K, T, s);
+        if (S == 2) return tc::launch<16, 4, 8, 2>(Wq, Wd, Xq, Xd, Resid, resid_ld, Y, M, K, T, s);
+        variant = 1;
+    }
+    if (variant == 1) return tc::launch<16, 4, 8, 1>(Wq, Wd, Xq, Xd, Resid, resid_ld, Y, M, K, T, s);
+    if (variant == 2) return tc::launch<32, 1, 8, 1>(Wq, Wd, Xq, Xd, Resid, resid_ld, Y, M, K, T, s);
+    if (variant == 3) return tc::launch<16, 4, 16, 1>(Wq, Wd, Xq, Xd, Resid, resid_ld, Y, M, K, T, s);
     set_error("lt_q8_gemm_tc: unknown variant %d", variant);
     return LT_ERR_INVALID;
 }

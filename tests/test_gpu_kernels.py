@@ -174,6 +174,22 @@ def gpu_gemm_tc(dWq, dWd, dXq, dXd, M, K, T, variant, resid=None, resid_ld=0):
     return y
 
 
+@pytest.mark.parametrize("M,K,T", [(128, 128, 9), (300, 896, 17), (200, 4864, 33), (130, 14336, 16), (1280, 4096, 70), (3100, 4864, 121)])
+def test_tensor_core_gemm_with_shared_tiles_bit_exact(oracle, M, K, T):
+    """Few tiles: clusters of two and four CTAs share the blocks of a tile, down to CTAs without a block, over one and
+    several tiles per cluster."""
+    Wq, Wd, x = synth.gemv_case(M, K, T=T, seed=T + 7)
+    xq, xd = gpu_quant(x, rows=T)
+    dWq, dWd = dev(Wq), dev(Wd)
+    want = oracle.q8_gemm(Wq, Wd, host(xq), host(xd, np.uint16), M, K, T)
+    y = host(gpu_gemm_tc(dWq, dWd, xq, xd, M, K, T, 0)).reshape(T, M)
+    assert np.array_equal(bits(y), bits(want))
+    R = np.random.default_rng(3).standard_normal((T, M)).astype(np.float32)
+    y = host(gpu_gemm_tc(dWq, dWd, xq, xd, M, K, T, 0, resid=dev(R), resid_ld=M)).reshape(T, M)
+    assert np.array_equal(bits(y), bits(want + R))
+    assert _lib.device_status() == set()
+
+
 @pytest.mark.parametrize("variant", [1, 2, 3])
 @pytest.mark.parametrize("M,K,T", [(128, 128, 16), (128, 896, 16), (896, 896, 64), (300, 4864, 33), (1152, 896, 70),
                                    (256, 4096, 5), (200, 14336, 17), (4864, 896, 257)])
