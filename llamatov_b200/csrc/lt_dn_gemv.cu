@@ -2,6 +2,9 @@
 // the fp32 vector into the matrix's element type itself (cast, RMS norm over groups, gate), so that norm, gate and
 // linear are one launch.  A warp owns pairs of rows (n, n + 1; gate n and its up row; or the one kind, then the other) and keeps two rows x U 16-byte
 // loads per lane in flight; the first batch of weights is requested before the input is touched.
+// Matrices of few long rows (output projections) have fewer pairs than the GPU has places for warps, and what is in
+// flight then bounds them: 2, 4 or 8 warps of a CTA share a pair, each takes every ws-th batch of its rows, and their sums
+// are added in order.  (M x K: 896 x 6656 fp32 12.0 us, now 7.9; 2048 x 8192 bf16 10.6, now 9.1; 300 x 4096 4.1, now 3.2.)
 #include "lt_dn_common.cuh"
 
 namespace lt {
@@ -12,6 +15,7 @@ struct GemvP {
     void* Y;
     int M, K, ldw, npair;
     int nstore, mstore;      // pairs of stored rows and those rows; the pairs that follow are gate and up
+    int ws;                  // warps that share a pair; more than one only where every pair has its own warps
     lt_dn_prologue pro;
     lt_dn_epilogue epi;
 };
@@ -129,14 +133,18 @@ __device__ __forceinline__ void make_input(const lt_dn_prologue& p, int K, float
     }
 }
 
-template <typename T>
+template <typename T, bool SHARED>     // SHARED: P.ws > 1 warps per pair
 __global__ void __launch_bounds__(GV_THREADS, 2) k_gemv(const __grid_constant__ GemvP P) {
     extern __shared__ __align__(16) float4 xs[];
     __shared__ float sred[GV_THREADS / 32];
+    __shared__ float2 spart[SHARED ? GV_THREADS / 32 : 1];
     constexpr int N = Vec<T>::N;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int nvec = P.K / N, nquad = P.K >> 2;
-    const int gw = blockIdx.x * (GV_THREADS / 32) + warp, nw = gridDim.x * (GV_THREADS / 32);
+    const int ws = SHARED ? P.ws : 1;
+    const int per_cta = GV_THREADS / 32 / ws, part = warp % ws;
+    const int gw = blockIdx.x * per_cta + warp / ws, nw = gridDim.x * per_cta;
+    const int first = part * 32 * GV_U, stride = ws * 32 * GV_U;     // 16-byte units of a row: this warp's batches
     const uint4 zero = make_uint4(0, 0, 0, 0);
 
     uint4 buf[2][GV_U];
@@ -168,7 +176,7 @@ __global__ void __launch_bounds__(GV_THREADS, 2) k_gemv(const __grid_constant__ 
     int pr = gw, r0 = 0, r1 = 0;
     if (pr < P.npair) {
         rows_of(pr, r0, r1);
-        fetch(r0, r1, 0);
+        fetch(r0, r1, first);
     }
     make_input<T>(P.pro, P.K, xs, sred);
     __syncthreads();
@@ -176,17 +184,17 @@ __global__ void __launch_bounds__(GV_THREADS, 2) k_gemv(const __grid_constant__ 
     for (; pr < P.npair; pr += nw) {
         float acc0 = 0.0f, acc1 = 0.0f;
         const int c0 = r0, c1 = r1;
-        for (int base = 0; base < nvec; base += 32 * GV_U) {
+        for (int base = first; base < nvec; base += stride) {
             uint4 w[2][GV_U];
 #pragma unroll
             for (int u = 0; u < GV_U; u++) {
                 w[0][u] = buf[0][u];
                 w[1][u] = buf[1][u];
             }
-            if (base + 32 * GV_U < nvec) fetch(c0, c1, base + 32 * GV_U);
+            if (base + stride < nvec) fetch(c0, c1, base + stride);
             else if (pr + nw < P.npair) {
                 rows_of(pr + nw, r0, r1);
-                fetch(r0, r1, 0);
+                fetch(r0, r1, first);
             }
 #pragma unroll
             for (int u = 0; u < GV_U; u++) {
@@ -209,6 +217,15 @@ __global__ void __launch_bounds__(GV_THREADS, 2) k_gemv(const __grid_constant__ 
         }
         acc0 = warp_sum(acc0);
         acc1 = warp_sum(acc1);
+        if (SHARED) {            // the one pair of these warps: the first of them finishes it
+            if (lane == 0) spart[warp] = make_float2(acc0, acc1);
+            asm volatile("bar.sync %0, %1;" ::"r"(1 + warp / ws), "r"(ws * 32) : "memory");
+            if (part != 0) return;
+            for (int i = 1; i < ws; i++) {
+                acc0 += spart[warp + i].x;
+                acc1 += spart[warp + i].y;
+            }
+        }
         if (pr >= P.nstore) {
             if (lane == 0) glu_store<T>(P.epi, P.epi.kind == LT_DN_GLU ? P.Y : P.epi.y2, c0 - P.mstore, acc0, acc1);
         } else if (lane < 2 && (lane == 0 || c1 != c0)) {
@@ -262,13 +279,21 @@ extern "C" int lt_dn_gemv(const void* W, int ldw, void* Y, int f32, int M, int K
     P.npair = P.nstore + M - P.mstore;
     static PerDeviceOnce once;
     if (once.first()) {
-        LT_CUDA(cudaFuncSetAttribute(k_gemv<bf16>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
-        LT_CUDA(cudaFuncSetAttribute(k_gemv<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
+        LT_CUDA(cudaFuncSetAttribute(k_gemv<bf16, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
+        LT_CUDA(cudaFuncSetAttribute(k_gemv<bf16, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
+        LT_CUDA(cudaFuncSetAttribute(k_gemv<float, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
+        LT_CUDA(cudaFuncSetAttribute(k_gemv<float, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
     }
     const int per = smem <= 100 * 1024 ? 2 : 1;
-    const int need = (P.npair + GV_THREADS / 32 - 1) / (GV_THREADS / 32);
+    // warps per pair: as many as the resident CTAs have for every pair, each with at least one whole batch
+    const long warps = (long)per * sm_count() * (GV_THREADS / 32);
+    const int batches = K / (f32 ? 4 : 8) / (32 * GV_U);
+    P.ws = 1;
+    while (P.ws < GV_THREADS / 32 && 2L * P.ws * P.npair <= warps && 2 * P.ws <= batches) P.ws *= 2;
+    const int per_cta = GV_THREADS / 32 / P.ws;
+    const int need = (P.npair + per_cta - 1) / per_cta;
     const int grid = need < per * sm_count() ? need : per * sm_count();
-    if (f32) k_gemv<float><<<grid, GV_THREADS, smem, (cudaStream_t)stream>>>(P);
-    else k_gemv<bf16><<<grid, GV_THREADS, smem, (cudaStream_t)stream>>>(P);
+    void (*kern)(GemvP) = f32 ? (P.ws > 1 ? k_gemv<float, true> : k_gemv<float, false>) : (P.ws > 1 ? k_gemv<bf16, true> : k_gemv<bf16, false>);
+    kern<<<grid, GV_THREADS, smem, (cudaStream_t)stream>>>(P);
     return check_launch("lt_dn_gemv");
 }

@@ -394,3 +394,23 @@ def test_fp32_linear_with_parts_of_k(M, K, T):
     e = P.epilogue(_lib.DN_GLU, out_f32=True)
     _lib.call("lt_dn_linear", W.data_ptr(), K, X.data_ptr(), K, Z.data_ptr(), M, 1, M, K, T, ctypes.byref(e), 0, stream())
     _close(_np(Z), L.gelu_tanh(v[:, :M]) * v[:, M:], 6 * tol)
+
+
+@pytest.mark.parametrize("f32", [0, 1])
+@pytest.mark.parametrize("M,K", [(3, 2048), (300, 4104), (2047, 2064), (700, 6656), (1200, 1032)])
+def test_gemv_rows_shared_by_warps(f32, M, K):
+    """Few rows: two, four and eight warps per pair of rows, an odd last row, ragged last batches; residual and gated."""
+    W, x = _t((2 * M, K), 16, f32, K ** -0.5), torch.randn(K).cuda()
+    xr = _np(x.to(DT[f32]))
+    v = _np(W) @ xr
+    tol = 2e-6 * K ** 0.5                    # fp32 sums of exact products in both types
+    ls, Y = torch.randn(M).cuda(), torch.randn(M).cuda()
+    y0 = _np(Y)
+    e = P.epilogue(_lib.DN_RESID, ls=ls)
+    pro = P.cast_input(x.data_ptr(), K)
+    _lib.call("lt_dn_gemv", W.data_ptr(), K, Y.data_ptr(), f32, M, K, ctypes.byref(pro), ctypes.byref(e), stream())
+    _close(_np(Y), y0 + v[:M] * _np(ls), 3 * tol)
+    e = P.epilogue(_lib.DN_GLU, out_f32=True)
+    Z = torch.empty(M, device="cuda")
+    _lib.call("lt_dn_gemv", W.data_ptr(), K, Z.data_ptr(), f32, M, K, ctypes.byref(pro), ctypes.byref(e), stream())
+    _close(_np(Z), L.gelu_tanh(v[:M]) * v[M:], 6 * tol)
