@@ -545,7 +545,7 @@ static int launch(const int8_t* Wq, const uint16_t* Wd, const int8_t* Xq, const 
     rc = make_map(&tmX, Xq, T, K, CB * 32, NT);
     if (rc != LT_OK) return rc;
     // as many stages as fit: a chunk of 18 KB is on its way for a microsecond or two (4 stages -> 8: 28672 x 4096 x 512
-    // 727 -> 684 us, 128256 x 4096 x 32 210 -> 204, narrow batches within 3 % either way)
+    // 727 -> 684 us, 128256 x 4096 x 32 210 -> 204, narrow batches within 6 % either way)
     const size_t rest = 1024 + 1024 + C::XCHG + (size_t)nb * NT * 4;
     int nstage = C::NSTAGE_MIN;
     while (nstage < 8 && rest + (size_t)(nstage + 2) * C::STAGE <= 220 * 1024) nstage += 2;
