@@ -3,8 +3,11 @@
 // linear are one launch.  A warp owns pairs of rows (n, n + 1; gate n and its up row; or the one kind, then the other) and keeps two rows x U 16-byte
 // loads per lane in flight; the first batch of weights is requested before the input is touched.
 // Matrices of few long rows (output projections) have fewer pairs than the GPU has places for warps, and what is in
-// flight then bounds them: 2, 4 or 8 warps of a CTA share a pair, each takes every ws-th batch of its rows, and their sums
-// are added in order.  (M x K: 896 x 6656 fp32 12.0 us, now 7.9; 2048 x 8192 bf16 10.6, now 9.1; 300 x 4096 4.1, now 3.2.)
+// flight then bounds them: 2, 4 or 8 warps of a CTA share a pair and each takes every ws-th batch of its rows.  The lanes'
+// running sums go from warp to warp with the batches, so that every sum is the chain of products that one warp makes alone
+// and a row's bits do not depend on how many rows its matrix has.
+// (M x K: 896 x 6656 fp32 11.8 us with a warp per pair, now 7.6; 896 x 4864 fp32 9.6, 6.3; 2048 x 8192 bf16 10.3, 9.0;
+// 300 x 4096 bf16 4.1, 3.7.)
 #include "lt_dn_common.cuh"
 
 namespace lt {
@@ -137,7 +140,7 @@ template <typename T, bool SHARED>     // SHARED: P.ws > 1 warps per pair
 __global__ void __launch_bounds__(GV_THREADS, 2) k_gemv(const __grid_constant__ GemvP P) {
     extern __shared__ __align__(16) float4 xs[];
     __shared__ float sred[GV_THREADS / 32];
-    __shared__ float2 spart[SHARED ? GV_THREADS / 32 : 1];
+    __shared__ float2 ssum[SHARED ? GV_THREADS / 64 : 1][32];        // running sums of a pair, on their way between its warps
     constexpr int N = Vec<T>::N;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int nvec = P.K / N, nquad = P.K >> 2;
@@ -183,6 +186,7 @@ __global__ void __launch_bounds__(GV_THREADS, 2) k_gemv(const __grid_constant__ 
 
     for (; pr < P.npair; pr += nw) {
         float acc0 = 0.0f, acc1 = 0.0f;
+        bool last = true;
         const int c0 = r0, c1 = r1;
         for (int base = first; base < nvec; base += stride) {
             uint4 w[2][GV_U];
@@ -192,9 +196,29 @@ __global__ void __launch_bounds__(GV_THREADS, 2) k_gemv(const __grid_constant__ 
                 w[1][u] = buf[1][u];
             }
             if (base + stride < nvec) fetch(c0, c1, base + stride);
-            else if (pr + nw < P.npair) {
+            else if (!SHARED && pr + nw < P.npair) {
                 rows_of(pr + nw, r0, r1);
                 fetch(r0, r1, first);
+            }
+            auto x_of = [&](int i, float (&x)[N]) {
+#pragma unroll
+                for (int j = 0; j < N / 4; j++) {
+                    const float4 q = xs[N == 8 ? j * (nquad >> 1) + i : i];
+                    x[4 * j] = q.x; x[4 * j + 1] = q.y; x[4 * j + 2] = q.z; x[4 * j + 3] = q.w;
+                }
+            };
+            float xb[SHARED ? GV_U : 1][N];      // read ahead of the wait, which the chain passes through
+            if (SHARED) {
+#pragma unroll
+                for (int u = 0; u < GV_U; u++) {
+                    const int i = base + u * 32 + lane;
+                    x_of(i < nvec ? i : 0, xb[SHARED ? u : 0]);
+                }
+            }
+            if (SHARED && base > 0) {    // the batch before this one is the neighbour's
+                asm volatile("bar.sync %0, 64;" ::"r"(1 + warp) : "memory");
+                acc0 = ssum[warp / ws][lane].x;
+                acc1 = ssum[warp / ws][lane].y;
             }
 #pragma unroll
             for (int u = 0; u < GV_U; u++) {
@@ -203,29 +227,24 @@ __global__ void __launch_bounds__(GV_THREADS, 2) k_gemv(const __grid_constant__ 
                 float f0[N], f1[N], x[N];
                 Vec<T>::unpack(w[0][u], f0);
                 Vec<T>::unpack(w[1][u], f1);
-#pragma unroll
-                for (int j = 0; j < N / 4; j++) {
-                    const float4 q = xs[N == 8 ? j * (nquad >> 1) + i : i];
-                    x[4 * j] = q.x; x[4 * j + 1] = q.y; x[4 * j + 2] = q.z; x[4 * j + 3] = q.w;
-                }
+                if (!SHARED) x_of(i, x);
 #pragma unroll
                 for (int j = 0; j < N; j++) {
-                    acc0 = fmaf(f0[j], x[j], acc0);
-                    acc1 = fmaf(f1[j], x[j], acc1);
+                    acc0 = fmaf(f0[j], SHARED ? xb[SHARED ? u : 0][j] : x[j], acc0);
+                    acc1 = fmaf(f1[j], SHARED ? xb[SHARED ? u : 0][j] : x[j], acc1);
+                }
+            }
+            if (SHARED) {
+                last = base + 32 * GV_U >= nvec;
+                if (!last) {
+                    ssum[warp / ws][lane] = make_float2(acc0, acc1);
+                    asm volatile("bar.arrive %0, 64;" ::"r"(1 + warp - part + (part + 1) % ws) : "memory");
                 }
             }
         }
+        if (SHARED && !last) return;     // the one pair of these warps: who has its last batch finishes it
         acc0 = warp_sum(acc0);
         acc1 = warp_sum(acc1);
-        if (SHARED) {            // the one pair of these warps: the first of them finishes it
-            if (lane == 0) spart[warp] = make_float2(acc0, acc1);
-            asm volatile("bar.sync %0, %1;" ::"r"(1 + warp / ws), "r"(ws * 32) : "memory");
-            if (part != 0) return;
-            for (int i = 1; i < ws; i++) {
-                acc0 += spart[warp + i].x;
-                acc1 += spart[warp + i].y;
-            }
-        }
         if (pr >= P.nstore) {
             if (lane == 0) glu_store<T>(P.epi, P.epi.kind == LT_DN_GLU ? P.Y : P.epi.y2, c0 - P.mstore, acc0, acc1);
         } else if (lane < 2 && (lane == 0 || c1 != c0)) {
@@ -285,11 +304,14 @@ extern "C" int lt_dn_gemv(const void* W, int ldw, void* Y, int f32, int M, int K
         LT_CUDA(cudaFuncSetAttribute(k_gemv<float, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
     }
     const int per = smem <= 100 * 1024 ? 2 : 1;
-    // warps per pair: as many as the resident CTAs have for every pair, each with at least one whole batch
+    // warps per pair: as many as the resident CTAs have for every pair, each with at least one whole batch.  A bf16 batch is
+    // twice the products of an fp32 one for the same bytes, and the chain through the warps then costs what is gained
+    // where rows are two or three batches (2048 x 2048 4.6 us with a warp per pair, 4.8 with two).
     const long warps = (long)per * sm_count() * (GV_THREADS / 32);
     const int batches = K / (f32 ? 4 : 8) / (32 * GV_U);
     P.ws = 1;
-    while (P.ws < GV_THREADS / 32 && 2L * P.ws * P.npair <= warps && 2 * P.ws <= batches) P.ws *= 2;
+    if (f32 || batches >= 4)
+        while (P.ws < GV_THREADS / 32 && 2L * P.ws * P.npair <= warps && 2 * P.ws <= batches) P.ws *= 2;
     const int per_cta = GV_THREADS / 32 / P.ws;
     const int need = (P.npair + per_cta - 1) / per_cta;
     const int grid = need < per * sm_count() ? need : per * sm_count();

@@ -414,3 +414,22 @@ def test_gemv_rows_shared_by_warps(f32, M, K):
     Z = torch.empty(M, device="cuda")
     _lib.call("lt_dn_gemv", W.data_ptr(), K, Z.data_ptr(), f32, M, K, ctypes.byref(pro), ctypes.byref(e), stream())
     _close(_np(Z), L.gelu_tanh(v[:M]) * v[M:], 6 * tol)
+
+
+@pytest.mark.parametrize("f32", [0, 1])
+@pytest.mark.parametrize("M,K", [(3, 2048), (300, 4104), (700, 6656), (1200, 2064), (2047, 8192)])
+def test_gemv_bits_do_not_depend_on_the_number_of_rows(f32, M, K):
+    """Warps that share a pair of rows (few rows) add the products in the order of a warp that has the pair to itself."""
+    many = 5200                              # enough pairs that no warps share one
+    W, x = _t((2 * many, K), 16, f32, K ** -0.5), torch.randn(K).cuda()
+    R = torch.randn(many).cuda()
+    pro = P.cast_input(x.data_ptr(), K)
+    few = torch.cat([W[:M], W[many:many + M]])
+    for epi, kw in ((_lib.DN_RESID, {}), (_lib.DN_GLU, dict(out_f32=True))):
+        out = []
+        for w, n in ((few, M), (W, many)):
+            Y = R[:n].clone()
+            e = P.epilogue(epi, ls=R, **kw) if epi == _lib.DN_RESID else P.epilogue(epi, **kw)
+            _lib.call("lt_dn_gemv", w.data_ptr(), K, Y.data_ptr(), f32, n, K, ctypes.byref(pro), ctypes.byref(e), stream())
+            out.append(_np(Y[:M]))
+        assert np.array_equal(*out), epi
