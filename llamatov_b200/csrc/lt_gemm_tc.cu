@@ -27,9 +27,11 @@
 // Split rows of blocks (S > 1): a cluster of S CTAs shares a tile, CTA r visits the groups g = r mod S, a whole subtree of
 // the tree; the levels across those subtrees and inside a group are added by the CTA that finishes a column, from all
 // CTAs' partials in its shared memory.  Small batches need it: a matrix of 4096 rows has 32 row tiles for 148 SMs
-// (4096 x 14336, 24 columns: 64 CTAs 57 us, 128 CTAs 37 us; 9 columns: 32 CTAs 67 us, 128 CTAs 31 us).
+// (4096 x 14336, 24 columns: 64 CTAs 55 us, 128 CTAs 34 us; 9 columns: 32 CTAs 66 us, 128 CTAs 28 us).
 // Every wait is bounded: after the limit a CTA sets LT_STATUS_WAIT_TIMEOUT, all its later waits
 // return at once, it drains and frees its tensor memory.
+#include <atomic>
+
 #include "lt_tc.cuh"
 
 namespace lt {
@@ -166,12 +168,8 @@ k_q8_gemm_tc(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CU
     auto group = [&](int gi) {   // the gi-th group this CTA visits
         return rank + S * (LV > 0 ? (int)(__brev((unsigned)gi) >> (32 - (LV > 0 ? LV : 1))) : 0);
     };
-    unsigned chunks = 0;         // of a tile, in this CTA
-#pragma unroll
-    for (int gi = 0; gi < G; gi++) {
-        const int b0 = CB * group(gi);
-        chunks += b0 < nb ? (unsigned)((nb - b0 + 31) >> 5) : 0u;
-    }
+    // of a tile, in this CTA: every S-th chunk
+    const unsigned chunks = (unsigned)((nb / CB + S - 1 - rank) / S);
     volatile int* abort_flag = &B->abort_flag;
 
     if (tid == 0) {
@@ -531,7 +529,67 @@ static int sm_count() {
     int dev = 0, sms = 148;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    return sms < 4 ? 4 : sms;
+    return sms < 1 ? 1 : sms;
+}
+
+// ---- how many CTAs share a 16-column tile
+// A tile of c chunks costs a round of CTAs, in microseconds (28 shapes from 128 x 512 to 16384 x 7168, 9 to 1500 columns):
+// alone 0.455 c + 1; two CTAs 0.5 c / 2 + 3; four 0.55 c / 4 + 4 (the exchange, and pairs that share what the L2 delivers).
+// 4096 x 14336: 9 columns 66 us alone, 37 with two, 28 with four; 24 columns 55, 34, 47; 33 columns 53, 65, 68; 96 columns
+// 108, 92, 134; 896 x 896: 6.3, 6.8, 7.3.  Four CTAs pay only in a single round, as measured: with more, two are better.
+// rooms[]: clusters of 2 and 4 that the GPU holds at once.  Four need SMs of one GPC, and the last few of the GPC counts that
+// are no multiple of four stay alone: 33 clusters on 148 SMs.  A launch takes no more clusters than that, since tiles are
+// dealt out in advance and the clusters that wait for a place would start when the others end.
+static double split_cost(int S, long tiles, int chunks, long room) {
+    if (room < 1) return 1e30;
+    const long rounds = (tiles + room - 1) / room;
+    if (S == 4 && rounds > 1) return 1e30;
+    const double c = (double)((chunks + S - 1) / S);
+    return (double)rounds * (S == 1 ? 0.455 * c + 1.0 : (S == 2 ? 0.5 * c + 3.0 : 0.55 * c + 4.0));
+}
+static size_t split_smem(int nb) {   // the exchange buffer of S = 4 is half that of 2
+    using C = Cfg<16, 4, 8, 2>;
+    return (size_t)1024 + C::NSTAGE_MIN * C::STAGE + 1024 + C::XCHG + (size_t)nb * 64;
+}
+static int choose_split(int M, int K, int T, int sms, int room2, int room4) {
+    const int nb = K / 32, chunks = nb / 4;
+    const long tiles = (long)((M + TM - 1) / TM) * ((T + 15) / 16);
+    if (split_smem(nb) > 220 * 1024) return 1;
+    const long rooms[3] = {sms, room2, room4};
+    int best = 0;
+    for (int i = 1; i < 3; i++)
+        if (split_cost(1 << i, tiles, chunks, rooms[i]) < split_cost(1 << best, tiles, chunks, rooms[best])) best = i;
+    return 1 << best;
+}
+
+// CTAs (S = 1) or clusters of S CTAs that the current device holds at once, asked for once per device
+template <int NT, int CB, int EW, int S>
+static int room() {
+    static std::atomic<int> known[64];
+    int dev = 0;
+    if (S == 1 || cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return sm_count() / S;
+    int n = known[dev].load(std::memory_order_relaxed);
+    if (n > 0) return n;
+    if (cudaFuncSetAttribute(k_q8_gemm_tc<NT, CB, EW, S>, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024) != cudaSuccess) {
+        cudaGetLastError();
+        return 0;
+    }
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)(sm_count() / S * S));
+    cfg.blockDim = dim3(Cfg<NT, CB, EW, S>::THREADS);
+    cfg.dynamicSmemBytes = 220 * 1024;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = S;
+    at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    if (cudaOccupancyMaxActiveClusters(&n, k_q8_gemm_tc<NT, CB, EW, S>, &cfg) != cudaSuccess) {
+        cudaGetLastError();
+        return 0;
+    }
+    known[dev].store(n, std::memory_order_relaxed);
+    return n;
 }
 
 template <int NT, int CB, int EW, int S>
@@ -563,9 +621,10 @@ static int launch(const int8_t* Wq, const uint16_t* Wd, const int8_t* Xq, const 
     P.row_tiles = (M + TM - 1) / TM;
     P.t_tiles = (T + NT - 1) / NT;
     const long tiles = (long)P.row_tiles * P.t_tiles;
-    const int room = sm_count() / S;
+    const int most = room<NT, CB, EW, S>();
+    LT_REQUIRE(most > 0, "lt_q8_gemm_tc: this device has no room for clusters of %d", S);
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)((tiles < room ? tiles : room) * S));
+    cfg.gridDim = dim3((unsigned)((tiles < most ? tiles : most) * S));
     cfg.blockDim = dim3(C::THREADS);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = s;
@@ -578,27 +637,6 @@ static int launch(const int8_t* Wq, const uint16_t* Wd, const int8_t* Xq, const 
         cfg.numAttrs = 1;
     }
     return check_launch("lt_q8_gemm_tc", 1, cudaLaunchKernelEx(&cfg, k_q8_gemm_tc<NT, CB, EW, S>, tmW, tmX, P));
-}
-
-// How many CTAs share a 16-column tile: the split whose busiest CTA has least to do.  A tile costs a CTA its chunks and
-// a fixed part, larger with the exchange (in chunks of about half a microsecond, from 4096 x 4096 and 4096 x 14336 at 16
-// and 32 columns).  Clusters of four get a place only where a GPC has four SMs free: 32 of them are counted on.
-static int choose_split(int M, int K, int T) {
-    const int sms = sm_count(), nb = K / 32;
-    const long tiles = (long)((M + TM - 1) / TM) * ((T + 15) / 16);
-    if ((size_t)1024 + Cfg<16, 4, 8, 2>::NSTAGE_MIN * Cfg<16, 4, 8, 2>::STAGE + 1024 + Cfg<16, 4, 8, 2>::XCHG + (size_t)nb * 64 > 220 * 1024) return 1;
-    int best = 1;
-    double best_cost = 0.0;
-    for (int S = 1; S <= 4; S *= 2) {
-        const long room = S == 4 ? sms * 32 / 148 : sms / S;
-        const long rounds = (tiles + room - 1) / room;
-        const double cost = (double)rounds * ((double)((nb / 4 + S - 1) / S) + (S == 1 ? 1.5 : 4.0));
-        if (S == 1 || cost < best_cost) {
-            best = S;
-            best_cost = cost;
-        }
-    }
-    return best;
 }
 
 }  // namespace tc
@@ -618,15 +656,19 @@ extern "C" int lt_q8_gemm_tc(const int8_t* Wq, const uint16_t* Wd, const int8_t*
                "lt_q8_gemm_tc: Y may alias Resid only when Resid has one row per column");
     cudaStream_t s = (cudaStream_t)stream;
     if (variant == 0) {
-        const int S = tc::choose_split(M, K, T);
-        if (S == 4) return tc::launch<16, 4, 8, 4>(Wq, Wd, Xq, Xd, Resid, resid_ld, Y, M, K, T, s);
-        if (S == 2) return tc::launch<16, 4, 8, 2>(Wq, Wd, Xq, Xd, Resid, resid_ld, Y, M, K, T, s);
-        variant = 1;
+        const int S = tc::choose_split(M, K, T, tc::sm_count(), tc::room<16, 4, 8, 2>(), tc::room<16, 4, 8, 4>());
+        variant = S == 4 ? 5 : (S == 2 ? 4 : 1);
     }
     if (variant == 1) return tc::launch<16, 4, 8, 1>(Wq, Wd, Xq, Xd, Resid, resid_ld, Y, M, K, T, s);
     if (variant == 2) return tc::launch<32, 1, 8, 1>(Wq, Wd, Xq, Xd, Resid, resid_ld, Y, M, K, T, s);
     if (variant == 3) return tc::launch<16, 4, 16, 1>(Wq, Wd, Xq, Xd, Resid, resid_ld, Y, M, K, T, s);
+    if (variant == 4) return tc::launch<16, 4, 8, 2>(Wq, Wd, Xq, Xd, Resid, resid_ld, Y, M, K, T, s);
+    if (variant == 5) return tc::launch<16, 4, 8, 4>(Wq, Wd, Xq, Xd, Resid, resid_ld, Y, M, K, T, s);
     set_error("lt_q8_gemm_tc: unknown variant %d", variant);
     return LT_ERR_INVALID;
+}
+
+extern "C" int lt_q8_gemm_tc_split(int M, int K, int T, int sms, int clusters2, int clusters4) {
+    return M > 0 && K > 0 && K % 128 == 0 && T > 0 && sms > 0 ? tc::choose_split(M, K, T, sms, clusters2, clusters4) : 0;
 }
 

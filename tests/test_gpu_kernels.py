@@ -176,8 +176,7 @@ def gpu_gemm_tc(dWq, dWd, dXq, dXd, M, K, T, variant, resid=None, resid_ld=0):
 
 @pytest.mark.parametrize("M,K,T", [(128, 128, 9), (300, 896, 17), (200, 4864, 33), (130, 14336, 16), (1280, 4096, 70), (3100, 4864, 121)])
 def test_tensor_core_gemm_with_shared_tiles_bit_exact(oracle, M, K, T):
-    """Few tiles: clusters of two and four CTAs share the blocks of a tile, down to CTAs without a block, over one and
-    several tiles per cluster."""
+    """Few tiles, the default form: alone, or clusters of two and four CTAs that share the blocks of a tile."""
     Wq, Wd, x = synth.gemv_case(M, K, T=T, seed=T + 7)
     xq, xd = gpu_quant(x, rows=T)
     dWq, dWd = dev(Wq), dev(Wd)
@@ -187,6 +186,24 @@ def test_tensor_core_gemm_with_shared_tiles_bit_exact(oracle, M, K, T):
     R = np.random.default_rng(3).standard_normal((T, M)).astype(np.float32)
     y = host(gpu_gemm_tc(dWq, dWd, xq, xd, M, K, T, 0, resid=dev(R), resid_ld=M)).reshape(T, M)
     assert np.array_equal(bits(y), bits(want + R))
+    assert _lib.device_status() == set()
+
+
+@pytest.mark.parametrize("variant", [4, 5])
+@pytest.mark.parametrize("M,K,T", [(128, 128, 9), (77, 256, 3), (300, 384, 40), (200, 4864, 17), (3100, 896, 121), (1300, 14336, 130),
+                                   (10000, 512, 33)])
+def test_tensor_core_gemm_with_two_and_four_ctas_per_tile(oracle, variant, M, K, T):
+    """CTAs without a block (one to three chunks of blocks), one tile per cluster, three to eight tiles per cluster, ragged rows
+    and columns; plain, with a bias and with a residual."""
+    Wq, Wd, x = synth.gemv_case(M, K, T=T, seed=T + variant)
+    xq, xd = gpu_quant(x, rows=T)
+    dWq, dWd = dev(Wq), dev(Wd)
+    want = oracle.q8_gemm(Wq, Wd, host(xq), host(xd, np.uint16), M, K, T)
+    rng = np.random.default_rng(4)
+    bias, R = rng.standard_normal(M).astype(np.float32), rng.standard_normal((T, M)).astype(np.float32)
+    for resid, ld, w in ((None, 0, want), (bias, 0, want + bias), (R, M, want + R)):
+        y = host(gpu_gemm_tc(dWq, dWd, xq, xd, M, K, T, variant, resid=None if resid is None else dev(resid), resid_ld=ld)).reshape(T, M)
+        assert np.array_equal(bits(y), bits(w))
     assert _lib.device_status() == set()
 
 
