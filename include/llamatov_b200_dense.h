@@ -88,12 +88,14 @@ int lt_dn_norm_rows(const float* x, int ldx, const int* rows, const float* w, in
 int lt_dn_concat_rows(const float* x, int ldx, int n1, const float* x2, int ldx2, int n2, void* y, int ldy, int f32, int T,
                       void* stream);
 
-/* Y[t][n] = epilogue((W x_t)[n]) for T rows.  bf16: tcgen05 tiles; fp32: CUDA cores.  `variant` 0 = choose the tile,
+/* Y[t][n] = epilogue((W x_t)[n]) for T rows.  bf16: tcgen05 tiles; fp32: CUDA cores, k summed in parts that depend on K
+ * alone, so that a row's bits do not depend on T.  `variant` 0 = choose the tile,
  * else the tile's token columns (32, 64, 128 or 256; 256 not for LT_DN_GLU). */
 int lt_dn_linear(const void* W, int ldw, const void* X, int ldx, void* Y, int ldy, int f32, int M, int K, int T,
                  const lt_dn_epilogue* h_epi, int variant, void* stream);
 
-/* The same for one row, whose input is made by a prologue in every CTA (norm, gate, cast). */
+/* The same for one row, whose input is made by a prologue in every CTA (norm, gate, cast); k is summed in 32 interleaved chains
+ * and a tree, whatever M is. */
 int lt_dn_gemv(const void* W, int ldw, void* Y, int f32, int M, int K, const lt_dn_prologue* h_pro,
                const lt_dn_epilogue* h_epi, void* stream);
 

@@ -288,17 +288,21 @@ static int launch_tc(const void* W, int ldw, const void* X, int ldx, GemmP P, cu
 
 // ---- fp32: every product and sum an fp32 fused multiply-add on the CUDA cores, which bound it.  64 weight rows x 8 MQ
 // tokens per CTA of 128 threads, a thread owns 4 rows (pairs of rows with GLU) x MQ tokens: 4 + MQ 16-byte reads of shared
-// memory per 16 MQ multiply-adds, three stages of 32 k filled by asynchronous copies.  A cluster of S CTAs shares a tile's
-// k, in equal contiguous parts added in rank order through distributed shared memory: a prompt of a few hundred tokens
-// has fewer tiles than the GPU has places for CTAs.  Against 4 x 4 per thread from single floats of one unbuffered stage,
-// no split (M x K x T): 896 x 6656 x 300 703 -> 121 us, 3640 x 896 x 300 109 -> 90, 8192 x 2048 x 512 758 -> 423 (56 % of
-// the multiply-adds' rate), 896 x 6656 x 45 700 -> 51.  Shorter chains of sums: errors equal or smaller.
+// memory per 16 MQ multiply-adds, three stages of 32 k filled by asynchronous copies.  k is summed in up to four contiguous
+// parts, added in order.  One CTA folds them in turn, or a cluster of as many CTAs takes one each and adds them through
+// distributed shared memory: a prompt of a few hundred tokens has fewer tiles than the GPU has places for CTAs.  The bits
+// are the same in every form, so a token's output does not depend on how many others share its pass.
+// Against 4 x 4 per thread from single floats of one unbuffered stage, one chain over k (M x K x T): 896 x 6656 x 300
+// 780 -> 113 us, 3640 x 896 x 300 117 -> 68, 8192 x 2048 x 512 gated 1075 -> 792, 896 x 6656 x 45 800 -> 49.  Shorter chains of
+// sums: errors against 64 bits about half.
 constexpr int F32_THREADS = 128, F32_BM = 64, F32_BK = 32, F32_ST = F32_BK + 4, F32_STAGES = 3;
 
-template <bool GLU, int MQ>
+template <bool GLU, int MQ, bool SHARED>
 struct F32Cfg {
     static constexpr int NG = GLU ? 2 : 1, BN = 8 * MQ, ROWS = NG * F32_BM + BN;
     static constexpr int SMEM = F32_STAGES * ROWS * F32_ST * 4;
+    // quads of k in flight (unrolled): as many as the registers of the resident CTAs leave room for, measured
+    static constexpr int QUADS = MQ == 4 && !SHARED ? 8 : (!GLU && (MQ == 4 || !SHARED) ? 4 : 2);
     static_assert(SMEM >= NG * 4 * MQ * F32_THREADS * 4, "the partials fit the stages");
 };
 
@@ -307,16 +311,17 @@ __device__ __forceinline__ void f32_cluster_sync() {
     asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
 
-template <bool GLU, int MQ>
+template <bool GLU, int MQ, bool SHARED>      // SHARED: a CTA per part of k, parts of them in a cluster; else a CTA folds all
 __global__ void __launch_bounds__(F32_THREADS)
-k_gemm_f32(const float* __restrict__ W, int ldw, const float* __restrict__ X, int ldx, int S, const __grid_constant__ GemmP P) {
-    using C = F32Cfg<GLU, MQ>;
+k_gemm_f32(const float* __restrict__ W, int ldw, const float* __restrict__ X, int ldx, int parts, const __grid_constant__ GemmP P) {
+    using C = F32Cfg<GLU, MQ, SHARED>;
     constexpr int NG = C::NG, BN = C::BN;
     extern __shared__ __align__(16) float f32_smem[];
     const int tid = threadIdx.x, n = tid & 15, m = tid >> 4;
-    const int n0 = blockIdx.x * F32_BM, t0 = blockIdx.y * BN, rank = blockIdx.z;
+    const int n0 = blockIdx.x * F32_BM, t0 = blockIdx.y * BN, rank = SHARED ? blockIdx.z : 0;
     const int nk = (P.K + F32_BK - 1) / F32_BK;
-    const int c0 = (int)((long)nk * rank / S), c1 = (int)((long)nk * (rank + 1) / S);
+    auto part_from = [&](int part) { return (int)((long)nk * part / parts); };     // first chunk of a part
+    const int c0 = SHARED ? part_from(rank) : 0, c1 = SHARED ? part_from(rank + 1) : nk;
 
     auto copy = [&](int c, int stage) {
         float* dst = f32_smem + stage * C::ROWS * F32_ST;
@@ -352,14 +357,27 @@ k_gemm_f32(const float* __restrict__ W, int ldw, const float* __restrict__ X, in
             for (int j = 0; j < 4; j++) acc[g][i][j] = 0.0f;
 #pragma unroll
     for (int s = 0; s < F32_STAGES - 1; s++) copy(c0 + s, s);
-    int stage = 0;
+    int stage = 0, part = 0, part_end = part_from(1);
+    // sums of the parts before this one wait in local memory: in registers they would halve the CTAs of an SM (zero, unknown
+    // to the compiler, keeps them there)
+    float before[SHARED ? 1 : NG * MQ * 4];
+    int zero = 0;
+    if (!SHARED) asm volatile("mov.u32 %0, 0;" : "=r"(zero));
+    auto add_before = [&]() {
+#pragma unroll
+        for (int g = 0; g < NG; g++)
+#pragma unroll
+            for (int i = 0; i < MQ; i++)
+#pragma unroll
+                for (int j = 0; j < 4; j++) acc[g][i][j] = before[SHARED ? 0 : (g * MQ + i) * 4 + j + zero] + acc[g][i][j];
+    };
     for (int c = c0; c < c1; c++) {
         asm volatile("cp.async.wait_group %0;" ::"n"(F32_STAGES - 2) : "memory");
         __syncthreads();                                   // chunk c is there, chunk c - 1 is used up
         copy(c + F32_STAGES - 1, stage == 0 ? F32_STAGES - 1 : stage - 1);
         const float4* w4 = (const float4*)(f32_smem + (stage * C::ROWS + n) * F32_ST);
         const float4* x4 = (const float4*)(f32_smem + (stage * C::ROWS + NG * F32_BM + m * MQ) * F32_ST);
-#pragma unroll 2
+#pragma unroll C::QUADS
         for (int k = 0; k < F32_BK / 4; k++) {
             float4 x[MQ];
 #pragma unroll
@@ -388,9 +406,24 @@ k_gemm_f32(const float* __restrict__ W, int ldw, const float* __restrict__ X, in
             }
         }
         stage = stage == F32_STAGES - 1 ? 0 : stage + 1;
+        if (!SHARED && c + 1 == part_end) {
+            if (part > 0) add_before();
+            if (++part < parts) {
+#pragma unroll
+                for (int g = 0; g < NG; g++)
+#pragma unroll
+                    for (int i = 0; i < MQ; i++)
+#pragma unroll
+                        for (int j = 0; j < 4; j++) {
+                            before[SHARED ? 0 : (g * MQ + i) * 4 + j + zero] = acc[g][i][j];
+                            acc[g][i][j] = 0.0f;
+                        }
+                part_end = part_from(part + 1);
+            }
+        }
     }
     asm volatile("cp.async.wait_all;" ::: "memory");
-    if (S > 1) {        // partials [g][token][row][thread]; every CTA adds up the tokens of its share
+    if (SHARED) {       // partials [g][token][row][thread]; every CTA adds up the tokens of its share
         __syncthreads();
 #pragma unroll
         for (int g = 0; g < NG; g++)
@@ -402,13 +435,13 @@ k_gemm_f32(const float* __restrict__ W, int ldw, const float* __restrict__ X, in
         const unsigned mine = smem_u32(f32_smem + tid);
 #pragma unroll
         for (int i = 0; i < MQ; i++) {
-            if (i * S / MQ != rank) continue;
+            if (i * parts / MQ != rank) continue;
 #pragma unroll
             for (int g = 0; g < NG; g++)
 #pragma unroll
                 for (int j = 0; j < 4; j++) {
                     float v = 0.0f;
-                    for (int r = 0; r < S; r++) {
+                    for (int r = 0; r < parts; r++) {
                         unsigned a;
                         float part;
                         asm volatile("mapa.shared::cluster.u32 %0, %1, %2;"
@@ -430,23 +463,24 @@ k_gemm_f32(const float* __restrict__ W, int ldw, const float* __restrict__ X, in
 #pragma unroll
         for (int i = 0; i < MQ; i++) {
             const int t = t0 + m * MQ + i;
-            if (t >= P.T || i * S / MQ != rank) continue;
+            if (t >= P.T || (SHARED && i * parts / MQ != rank)) continue;
             if (GLU) glu_store<float>(P.epi, P.Y, (long)t * P.ldy + row, acc[0][i][j], acc[NG - 1][i][j]);
             else epi_store<float>(P.epi, re, P.Y, t, P.ldy, row, acc[0][i][j]);
         }
     }
 }
 
-template <bool GLU, int MQ>
+// Parts of k that every output is added up from: of K alone, so that a token's bits do not depend on the pass it is in.
+static int f32_parts(int K) { return K >= 32 * 32 ? 4 : (K >= 16 * 32 ? 2 : 1); }
+
+template <bool GLU, int MQ, bool SHARED>
 static int launch_f32(const void* W, int ldw, const void* X, int ldx, const GemmP& P, cudaStream_t s) {
-    using C = F32Cfg<GLU, MQ>;
+    using C = F32Cfg<GLU, MQ, SHARED>;
     static PerDeviceOnce once;
-    if (once.first()) LT_CUDA(cudaFuncSetAttribute(k_gemm_f32<GLU, MQ>, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM));
+    if (once.first()) LT_CUDA(cudaFuncSetAttribute(k_gemm_f32<GLU, MQ, SHARED>, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM));
     const long gx = (P.M + F32_BM - 1) / F32_BM, gy = (P.T + C::BN - 1) / C::BN;
     LT_REQUIRE(gy <= 65535, "lt_dn_linear: T=%d too large", P.T);
-    // parts of k: until three CTAs per SM are there, each with at least eight chunks
-    int S = 1;
-    while (S < 4 && gx * gy * S < 3 * sm_count() && P.K / F32_BK / (2 * S) >= 8) S *= 2;
+    const int parts = f32_parts(P.K), S = SHARED ? parts : 1;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)gx, (unsigned)gy, (unsigned)S);
     cfg.blockDim = dim3(F32_THREADS);
@@ -457,9 +491,45 @@ static int launch_f32(const void* W, int ldw, const void* X, int ldx, const Gemm
     at[0].val.clusterDim.x = at[0].val.clusterDim.y = 1;
     at[0].val.clusterDim.z = (unsigned)S;
     cfg.attrs = at;
-    cfg.numAttrs = 1;
+    cfg.numAttrs = SHARED ? 1 : 0;
     return check_launch("lt_dn_linear", 1,
-                        cudaLaunchKernelEx(&cfg, k_gemm_f32<GLU, MQ>, (const float*)W, ldw, (const float*)X, ldx, S, P));
+                        cudaLaunchKernelEx(&cfg, k_gemm_f32<GLU, MQ, SHARED>, (const float*)W, ldw, (const float*)X, ldx, parts, P));
+}
+
+// The form with the least estimated time.  n CTAs together on an SM take a + b n us per chunk of 32 k each, and every round of
+// them o us beside that (first loads, epilogue, exchange between the CTAs of a cluster): fitted to 223 sizes (16 matrices from
+// 32 x 896 to 16384 x 1024, 2 to 2000 tokens), where the form chosen is 0.4 % off the fastest on average, 10 % at most.
+// Clusters lose another 8 % where they need several rounds, since a place for one is free only when all of its CTAs find one.
+// 896 x 6656, 2 tokens: 176 us with 32 tokens per CTA, 46 with k shared; 16384 x 1024, 1000 tokens: 903, 1095 and with 64
+// tokens per CTA 830, shared 1300; 2048 x 8192, 1000 tokens: 920, 960, 915, 879.
+struct F32Time { double a, b, o; };
+template <bool GLU, int MQ, bool SHARED>
+static double f32_time(const GemmP& P, const F32Time& t) {
+    using C = F32Cfg<GLU, MQ, SHARED>;
+    const int parts = f32_parts(P.K);
+    if ((SHARED && parts == 1) || ((long)P.T + C::BN - 1) / C::BN > 65535) return 1e30;
+    const int S = SHARED ? parts : 1, chunks = ((P.K + F32_BK - 1) / F32_BK + S - 1) / S;
+    const long ctas = (long)((P.M + F32_BM - 1) / F32_BM) * ((P.T + C::BN - 1) / C::BN) * S;
+    const long per_sm = (ctas + sm_count() - 1) / sm_count();
+    const int together = 227 * 1024 / (C::SMEM + 1024);
+    const long rounds = per_sm / together, rest = per_sm % together;
+    double us = (double)rounds * (chunks * (t.a + t.b * together) + t.o);
+    if (rest > 0) us += chunks * (t.a + t.b * (double)rest) + t.o;
+    return SHARED && per_sm > together ? 1.08 * us : us;
+}
+template <bool GLU>
+static int pick_f32(const void* W, int ldw, const void* X, int ldx, const GemmP& P, cudaStream_t s) {
+    const double us[4] = {f32_time<GLU, 4, false>(P, GLU ? F32Time{0.54, 0.70, 3.0} : F32Time{0.40, 0.43, 3.0}),
+                          f32_time<GLU, 4, true>(P, GLU ? F32Time{0.43, 0.81, 7.0} : F32Time{0.30, 0.46, 5.0}),
+                          f32_time<GLU, 8, false>(P, GLU ? F32Time{0.45, 1.50, 7.0} : F32Time{0.30, 0.84, 9.0}),
+                          f32_time<GLU, 8, true>(P, GLU ? F32Time{0.32, 1.60, 19.0} : F32Time{0.20, 0.95, 14.0})};
+    int form = 0;
+    for (int i = 1; i < 4; i++)
+        if (us[i] < us[form]) form = i;
+    if (form == 0) return launch_f32<GLU, 4, false>(W, ldw, X, ldx, P, s);
+    if (form == 1) return launch_f32<GLU, 4, true>(W, ldw, X, ldx, P, s);
+    if (form == 2) return launch_f32<GLU, 8, false>(W, ldw, X, ldx, P, s);
+    return launch_f32<GLU, 8, true>(W, ldw, X, ldx, P, s);
 }
 
 // tile width: fewest (waves x time of a tile); a tile costs its columns plus what does not shrink with them
@@ -503,12 +573,8 @@ extern "C" int lt_dn_linear(const void* W, int ldw, const void* X, int ldx, void
     GemmP P = {};
     P.Y = Y; P.M = M; P.K = K; P.T = T; P.ldy = ldy; P.epi = *h_epi; P.up_row = M;
     const bool glu = h_epi->kind == LT_DN_GLU;
-    if (f32) {
-        // 64 tokens per CTA while that gives every SM a tile, else 32 (half the reuse, twice the CTAs)
-        const bool wide = (long)((M + 63) / 64) * ((T + 63) / 64) >= sm_count();
-        if (glu) return wide ? launch_f32<true, 8>(W, ldw, X, ldx, P, s) : launch_f32<true, 4>(W, ldw, X, ldx, P, s);
-        return wide ? launch_f32<false, 8>(W, ldw, X, ldx, P, s) : launch_f32<false, 4>(W, ldw, X, ldx, P, s);
-    }
+    if (f32)
+        return glu ? pick_f32<true>(W, ldw, X, ldx, P, s) : pick_f32<false>(W, ldw, X, ldx, P, s);
     const int nt = variant ? variant : choose_nt(M, T, glu);
     if (glu) {
         LT_REQUIRE(nt <= 128, "lt_dn_linear: tiles of 256 tokens do not fit a gated pair");

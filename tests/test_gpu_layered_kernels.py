@@ -373,10 +373,12 @@ def test_window_edge_shows(f32, T):
         assert abs(o[t, 16 + 7] - (0.0 if sees else 4.0)) < 0.05, (t, o[t, 23])
 
 
-@pytest.mark.parametrize("M,K,T", [(70, 1096, 33), (65, 520, 1), (896, 2080, 31), (4800, 544, 130)])
+@pytest.mark.parametrize("M,K,T", [(70, 1096, 33), (65, 520, 1), (896, 2080, 31), (4800, 544, 130), (200, 136, 50), (1500, 520, 1100), (520, 1032, 700),
+                                   (1500, 136, 600), (200, 2088, 900)])
 def test_fp32_linear_with_parts_of_k(M, K, T):
-    """Few tiles of long rows: a cluster shares k (four and two parts, with a ragged last chunk, rows and tokens), every
-    epilogue; and enough tiles for the wide form.  Bound: 4 roundings' growth of a K-term fp32 sum of O(1) products."""
+    """k in one, two and four parts, in a cluster or in turn in one CTA, 32 and 64 tokens per CTA (on 148 SMs every form, plain
+    and gated), with ragged last chunks, rows and tokens; every epilogue.  Bound: 4 roundings' growth of a K-term fp32 sum
+    of O(1) products."""
     W, X = _t((2 * M, K), 8, 1, K ** -0.5), _t((T, K), 9, 1)
     tol = 2e-6 * K ** 0.5
     v = _np(X) @ _np(W).T
@@ -433,3 +435,18 @@ def test_gemv_bits_do_not_depend_on_the_number_of_rows(f32, M, K):
             _lib.call("lt_dn_gemv", w.data_ptr(), K, Y.data_ptr(), f32, n, K, ctypes.byref(pro), ctypes.byref(e), stream())
             out.append(_np(Y[:M]))
         assert np.array_equal(*out), epi
+
+
+@pytest.mark.parametrize("M,K", [(900, 1104), (70, 6656), (4864, 520), (8192, 1024)])
+def test_fp32_linear_bits_do_not_depend_on_the_other_tokens(M, K):
+    """A token alone in its pass, in passes of a few and of many hundred tokens: the same bits, plain and gated."""
+    W, X = _t((2 * M, K), 18, 1, K ** -0.5), _t((1000, K), 19, 1)
+    for epi in (None, _lib.DN_GLU):
+        def run(X):
+            Y = torch.empty(len(X), M, device="cuda")
+            e = P.epilogue(out_f32=True) if epi is None else P.epilogue(epi, out_f32=True)
+            _lib.call("lt_dn_linear", W.data_ptr(), K, X.data_ptr(), K, Y.data_ptr(), M, 1, M, K, len(X), ctypes.byref(e), 0, stream())
+            return Y
+        want = run(X)
+        for a, b in ((0, 1), (7, 10), (33, 66), (100, 200), (300, 620)):
+            assert torch.equal(run(X[a:b].clone()), want[a:b]), (epi, a, b)
