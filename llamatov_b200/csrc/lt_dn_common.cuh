@@ -162,18 +162,6 @@ __device__ __forceinline__ float warp_max(float v) {
     return v;
 }
 
-inline int sm_count() {
-    static int cache[64] = {0};
-    int dev = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 148;
-    if (cache[dev] == 0) {
-        int n = 148;
-        cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
-        cache[dev] = n;
-    }
-    return cache[dev];
-}
-
 // host checks shared by the launchers
 inline const char* epi_error(const lt_dn_epilogue* e) {
     if (e == nullptr) return "null epilogue";

@@ -9,8 +9,8 @@ namespace lt {
 
 // ------------------------------------------------------------------ quantiser
 // Four elements per thread: bound by the bytes (5 per element) once there are enough of them; a warp per block, one
-// element per lane (k_quant_q8_any, any alignment), issued four times the loads and stores and twice the divisions
-// (2048 x 4864: 29.6 us, now 18.5 us; 2048 x 896: 8.3, now 5.3).
+// element per lane (k_quant_q8_lane), issues four times the loads and stores and twice the divisions
+// (2048 x 4864: 29.6 us, 18.5 with four; 2048 x 896: 8.3, 5.3).
 __global__ void __launch_bounds__(256) k_quant_q8(const float* __restrict__ X, int8_t* __restrict__ Xq,
                                                   __half* __restrict__ Xd, long nblocks) {
     const long i = (long)blockIdx.x * 256 + threadIdx.x;      // quad of elements
@@ -25,8 +25,9 @@ __global__ void __launch_bounds__(256) k_quant_q8(const float* __restrict__ X, i
     ((char4*)Xq)[i] = q;
 }
 
-// one warp per 32-block, lane = element
-__global__ void __launch_bounds__(256) k_quant_q8_any(const float* __restrict__ X, int8_t* __restrict__ Xq,
+// One warp per 32-block, lane = element; any alignment.  Its chain of divisions is a quarter as long, which counts while every
+// block has a resident warp of its own (1 x 4864: 1.47 us, 1.53 with four elements per thread; 300 x 896: 1.70, 2.00).
+__global__ void __launch_bounds__(256) k_quant_q8_lane(const float* __restrict__ X, int8_t* __restrict__ Xq,
                                                    __half* __restrict__ Xd, long nblocks) {
     long b = (long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
     int lane = threadIdx.x & 31;
@@ -305,10 +306,11 @@ extern "C" int lt_quant_q8(const float* X, int8_t* Xq, uint16_t* Xd, int K, int 
     LT_REQUIRE(X && Xq && Xd, "lt_quant_q8: null pointer");
     LT_REQUIRE(K > 0 && K % 32 == 0 && rows > 0, "lt_quant_q8: K=%d must be a positive multiple of 32, rows=%d > 0", K, rows);
     long nblocks = (long)rows * (K / 32);
-    if (aligned16(X) && (reinterpret_cast<uintptr_t>(Xq) & 3u) == 0)
+    // more blocks than the SMs hold warps (64 each): 8192 blocks 1.88 us either way, 12288 2.37 and 2.11
+    if (nblocks > 64L * sm_count() && aligned16(X) && (reinterpret_cast<uintptr_t>(Xq) & 3u) == 0)
         k_quant_q8<<<(unsigned)((nblocks + 31) / 32), 256, 0, (cudaStream_t)stream>>>(X, Xq, (__half*)Xd, nblocks);
     else
-        k_quant_q8_any<<<(unsigned)((nblocks + 7) / 8), 256, 0, (cudaStream_t)stream>>>(X, Xq, (__half*)Xd, nblocks);
+        k_quant_q8_lane<<<(unsigned)((nblocks + 7) / 8), 256, 0, (cudaStream_t)stream>>>(X, Xq, (__half*)Xd, nblocks);
     return check_launch("lt_quant_q8");
 }
 

@@ -77,8 +77,8 @@ __global__ void k_add_len(int* len, int n, int max_seq) {
 
 // ------------------------------------------------------------------ silu * up -> quant, strided rows
 // Four elements per thread, eight threads per block: bound by its 9 bytes per element and by the exponential and the
-// divisions of silu and the quantiser.  A warp per block with one element per lane (k_silu_mul_quant_rows_any, any
-// alignment) had four times the instructions around them: 2048 rows of 4864, 53.7 us, now 28.7 us.
+// divisions of silu and the quantiser.  A warp per block with one element per lane (k_silu_mul_quant_rows_lane) has four times
+// the instructions around them: 2048 rows of 4864, 53.7 us, 28.7 with four.
 __global__ void __launch_bounds__(256) k_silu_mul_quant_rows(const float* __restrict__ G, const float* __restrict__ U, int ld,
                                                              int8_t* __restrict__ Xq, __half* __restrict__ Xd, int K, int rows) {
     chain_release();
@@ -97,8 +97,9 @@ __global__ void __launch_bounds__(256) k_silu_mul_quant_rows(const float* __rest
     if ((i & 7) == 0) Xd[i >> 3] = d;
 }
 
-__global__ void k_silu_mul_quant_rows_any(const float* __restrict__ G, const float* __restrict__ U, int ld,
-                                      int8_t* __restrict__ Xq, __half* __restrict__ Xd, int K, int rows) {
+// any alignment, and few blocks: a quarter of the chain of divisions (1 x 4864: 1.64 us, 1.75 with four; 150 x 896: 1.82, 2.11)
+__global__ void k_silu_mul_quant_rows_lane(const float* __restrict__ G, const float* __restrict__ U, int ld,
+                                           int8_t* __restrict__ Xq, __half* __restrict__ Xd, int K, int rows) {
     chain_release();
     chain_wait();
     const int nb = K >> 5;
@@ -845,11 +846,12 @@ extern "C" int lt_silu_mul_quant_rows(const float* g, const float* u, int ld, in
     LT_REQUIRE(g && u && Xq && Xd, "lt_silu_mul_quant_rows: null pointer");
     LT_REQUIRE(K > 0 && K % 32 == 0 && rows > 0 && ld >= K, "lt_silu_mul_quant_rows: K=%d rows=%d ld=%d", K, rows, ld);
     const long blocks32 = (long)rows * (K / 32);
-    const bool quads = aligned16(g) && aligned16(u) && ld % 4 == 0 && (reinterpret_cast<uintptr_t>(Xq) & 3u) == 0;
+    // more than 40 blocks per SM: 5120 blocks 2.16 us, 2.21 with four elements per thread, 6144 2.46 and 2.25
+    const bool quads = blocks32 > 40L * sm_count() && aligned16(g) && aligned16(u) && ld % 4 == 0 && (reinterpret_cast<uintptr_t>(Xq) & 3u) == 0;
     const cudaError_t e =
         quads ? launch_chained(k_silu_mul_quant_rows, dim3((unsigned)((blocks32 + 31) / 32)), dim3(256), 0, (cudaStream_t)stream, g, u,
                                ld, Xq, (__half*)Xd, K, rows)
-              : launch_chained(k_silu_mul_quant_rows_any, dim3((unsigned)((blocks32 + 7) / 8)), dim3(256), 0, (cudaStream_t)stream, g, u,
+              : launch_chained(k_silu_mul_quant_rows_lane, dim3((unsigned)((blocks32 + 7) / 8)), dim3(256), 0, (cudaStream_t)stream, g, u,
                                ld, Xq, (__half*)Xd, K, rows);
     return check_launch("lt_silu_mul_quant_rows", 1, e);
 }

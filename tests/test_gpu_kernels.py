@@ -44,10 +44,10 @@ def test_quant_batched_rows(oracle):
         assert np.array_equal(host(xd, np.uint16).reshape(5, -1)[r], od.view(np.uint16))
 
 
-@pytest.mark.parametrize("K,rows", [(32, 1), (32, 31), (96, 33), (896, 5)])
+@pytest.mark.parametrize("K,rows", [(32, 1), (96, 33), (896, 5), (32, 6007), (4864, 63), (96, 3171)])
 def test_quantisers_of_four_elements_per_thread(K, rows):
-    """The vector forms give the bytes of the lane-per-element forms (taken for addresses off the 16-byte grid), with
-    NaNs, infinities and blocks of zeros among the values."""
+    """The vector forms (taken from 40 and 64 blocks per SM on) give the bytes of the lane-per-element forms (taken for fewer, and
+    for addresses off the 16-byte grid), with NaNs, infinities and blocks of zeros among the values."""
     rng = np.random.default_rng(K + rows)
     n = rows * K
 
