@@ -113,11 +113,10 @@ struct Params {
     int* status;
     int M, K, T;
     int row_tiles, t_tiles;
-    int nstage;     // stages of the ring, even, at most 8
     int resid_ld;   // 0: Resid[n] for every column (bias); else Resid[t * resid_ld + n]
 };
 
-template <int NT, int CB, int EW, int S>
+template <int NT, int CB, int EW, int S, int NST>      // NST: stages of the ring
 struct Cfg {
     static constexpr int CW = NT * 4 / EW;             // columns per epilogue thread
     static constexpr int G = 32 / CB / S;              // lane groups that a CTA of the cluster visits
@@ -129,7 +128,6 @@ struct Cfg {
     static constexpr int W_STAGE = CB * TM * 32;       // bytes: one stage = one chunk of CB blocks
     static constexpr int X_STAGE = CB * NT * 32;
     static constexpr int STAGE = W_STAGE + ((X_STAGE + 1023) / 1024) * 1024;
-    static constexpr int NSTAGE_MIN = CB == 4 ? 4 : (CB == 2 ? 6 : 8);
     static constexpr int SLOT_COLS = CB * NT;
     static constexpr int NSLOT = TMEM_COLS / SLOT_COLS;
     static constexpr int LB = CB * CW <= 16 ? CB : (CB >= 2 && CW <= 8 ? 2 : 1);   // blocks per TMEM round trip
@@ -148,20 +146,20 @@ struct Barriers {
     int next_start[32];   // per visiting position: first block of the next group that has blocks, -1 = none
 };
 
-template <int NT, int CB, int EW, int S>
-__global__ void __launch_bounds__(Cfg<NT, CB, EW, S>::THREADS, 1)
+template <int NT, int CB, int EW, int S, int NSTAGE>
+__global__ void __launch_bounds__(Cfg<NT, CB, EW, S, NSTAGE>::THREADS, 1)
 k_q8_gemm_tc(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUtensorMap tmX, const Params P) {
-    using C = Cfg<NT, CB, EW, S>;
+    using C = Cfg<NT, CB, EW, S, NSTAGE>;
     constexpr int CW = C::CW, G = C::G, LV = C::LV, NSLOT = C::NSLOT, LB = C::LB, MW = C::MW;
     extern __shared__ __align__(1024) unsigned char smem_raw[];
-    // 1024-byte aligned carve-up: stages (weights, then activations), barriers, activation scales
+    // 1024-byte aligned carve-up: stages (weights, then activations), barriers, exchange, activation scales
     unsigned char* base = (unsigned char*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
-    Barriers* B = (Barriers*)(base + P.nstage * C::STAGE);
+    Barriers* B = (Barriers*)(base + NSTAGE * C::STAGE);
     float* xchg = (float*)((unsigned char*)B + 1024);
     float* xs = (float*)((unsigned char*)xchg + C::XCHG);
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int nb = P.K >> 5, NSTAGE = P.nstage;
+    const int nb = P.K >> 5;
     const int tiles = P.row_tiles * P.t_tiles;
     const int rank = S > 1 ? (int)cluster_rank() : 0;
     const int tile_first = blockIdx.x / S, tile_step = gridDim.x / S;
@@ -172,25 +170,27 @@ k_q8_gemm_tc(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CU
     const unsigned chunks = (unsigned)((nb / CB + S - 1 - rank) / S);
     volatile int* abort_flag = &B->abort_flag;
 
-    if (tid == 0) {
-        for (int s = 0; s < NSTAGE; s++) {
-            mbar_init(&B->full[s], 1);
-            mbar_init(&B->empty[s], 1);
+    if (warp == 0) {   // a lane per barrier and per visiting position: one thread alone takes 0.2 us longer
+        if (lane < NSTAGE) {
+            mbar_init(&B->full[lane], 1);
+            mbar_init(&B->empty[lane], 1);
         }
-        for (int s = 0; s < NSLOT; s++) {
-            mbar_init(&B->tfull[s], 1);
-            mbar_init(&B->tempty[s], EW);
+        if (lane < NSLOT) {
+            mbar_init(&B->tfull[lane], 1);
+            mbar_init(&B->tempty[lane], EW);
         }
-        mbar_init(&B->xfull, 4 * S);
-        for (int s = 0; s < 4; s++) mbar_init(&B->xfree[s], EW);
-        B->abort_flag = 0;
-        for (int gi = 0; gi < G; gi++) {
+        if (S > 1 && lane < S) mbar_init(&B->xfree[lane], EW);
+        if (lane == 0) {
+            if (S > 1) mbar_init(&B->xfull, 4 * S);
+            B->abort_flag = 0;
+        }
+        if (lane < G) {
             int nxt = -1;
-            for (int gj = gi + 1; gj < G && nxt < 0; gj++) {
+            for (int gj = G - 1; gj > lane; gj--) {
                 const int b0 = CB * group(gj);
                 if (b0 < nb) nxt = b0;
             }
-            B->next_start[gi] = nxt;
+            B->next_start[lane] = nxt;
         }
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
@@ -212,23 +212,19 @@ k_q8_gemm_tc(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CU
     if (warp == EW) {
         // ------------------------------------------------------------------ producer
         if (lane == 0) {
-            int s = 0;             // stage of the next chunk
-            unsigned phase = 0;    // of its barriers
+            unsigned it = 0;   // chunks issued
             for (int tile = tile_first; tile < tiles; tile += tile_step) {
                 const int rt = tile / P.t_tiles, tt = tile - rt * P.t_tiles;
                 const int row0 = rt * TM, t0 = tt * NT;
                 for (int gi = 0; gi < G; gi++) {
                     const int g = group(gi);
-                    for (int b0 = CB * g; b0 < nb; b0 += 32) {
+                    for (int b0 = CB * g; b0 < nb; b0 += 32, it++) {
+                        const int s = it % NSTAGE;
                         unsigned char* st = base + s * C::STAGE;
-                        mbar_wait<64>(&B->empty[s], phase ^ 1, abort_flag, P.status);
+                        mbar_wait<64>(&B->empty[s], ((it / NSTAGE) & 1) ^ 1, abort_flag, P.status);
                         mbar_expect_tx(&B->full[s], C::W_STAGE + C::X_STAGE);
                         tma_load_2d(st, &tmW, b0 * 32, row0, &B->full[s]);
                         tma_load_2d(st + C::W_STAGE, &tmX, b0 * 32, t0, &B->full[s]);
-                        if (++s == NSTAGE) {
-                            s = 0;
-                            phase ^= 1;
-                        }
                     }
                 }
             }
@@ -246,10 +242,9 @@ k_q8_gemm_tc(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CU
             int my_tiles = 0;
             for (int tile = tile_first; tile < tiles; tile += tile_step) my_tiles++;
             const unsigned total = (unsigned)my_tiles * chunks;
-            unsigned s = (unsigned)(warp - (EW + 1)), phase = 0;     // stage of chunk it, phase of its barriers
-            for (unsigned it = s; it < total; it += MW) {
-                const unsigned slot = it % NSLOT;
-                mbar_wait<32>(&B->full[s], phase, abort_flag, P.status);
+            for (unsigned it = (unsigned)(warp - (EW + 1)); it < total; it += MW) {
+                const unsigned s = it % NSTAGE, slot = it % NSLOT;
+                mbar_wait<32>(&B->full[s], (it / NSTAGE) & 1, abort_flag, P.status);
                 mbar_wait<32>(&B->tempty[slot], ((it / NSLOT) & 1) ^ 1, abort_flag, P.status);
                 tc_fence_after();
                 // descriptors differ from the first stage's only in the start address (16-byte units)
@@ -261,11 +256,6 @@ k_q8_gemm_tc(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CU
                     mma_i8(d0 + i * NT, wd0 + 2 * i, xd0 + 2 * i, idesc);
                 mma_commit(&B->empty[s]);     // the stage may be refilled once these MMAs have read it
                 mma_commit(&B->tfull[slot]);  // and the slot holds the block sums
-                s += MW;
-                if (s >= (unsigned)NSTAGE) {
-                    s -= (unsigned)NSTAGE;
-                    phase ^= 1;
-                }
             }
         }
     } else {
@@ -525,13 +515,6 @@ static int make_map(CUtensorMap* m, const void* ptr, int rows, int K, int box_k,
     return LT_OK;
 }
 
-static int sm_count() {
-    int dev = 0, sms = 148;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    return sms < 1 ? 1 : sms;
-}
-
 // ---- how many CTAs share a 16-column tile
 // A tile of c chunks costs a round of CTAs, in microseconds (28 shapes from 128 x 512 to 16384 x 7168, 9 to 1500 columns):
 // alone 0.455 c + 1; two CTAs 0.5 c / 2 + 3; four 0.55 c / 4 + 4 (the exchange, and pairs that share what the L2 delivers).
@@ -547,14 +530,17 @@ static double split_cost(int S, long tiles, int chunks, long room) {
     const double c = (double)((chunks + S - 1) / S);
     return (double)rounds * (S == 1 ? 0.455 * c + 1.0 : (S == 2 ? 0.5 * c + 3.0 : 0.55 * c + 4.0));
 }
-static size_t split_smem(int nb) {   // the exchange buffer of S = 4 is half that of 2
-    using C = Cfg<16, 4, 8, 2>;
-    return (size_t)1024 + C::NSTAGE_MIN * C::STAGE + 1024 + C::XCHG + (size_t)nb * 64;
+// bytes of shared memory of a launch; a CTA may have MAX_SMEM
+constexpr size_t MAX_SMEM = 220 * 1024;
+template <int NT, int CB, int EW, int S, int NST>
+static size_t smem_bytes(int nb) {
+    using C = Cfg<NT, CB, EW, S, NST>;
+    return 1024 + (size_t)NST * C::STAGE + 1024 + C::XCHG + (size_t)nb * NT * 4;
 }
 static int choose_split(int M, int K, int T, int sms, int room2, int room4) {
     const int nb = K / 32, chunks = nb / 4;
     const long tiles = (long)((M + TM - 1) / TM) * ((T + 15) / 16);
-    if (split_smem(nb) > 220 * 1024) return 1;
+    if (smem_bytes<16, 4, 8, 2, 6>(nb) > MAX_SMEM) return 1;     // four need less
     const long rooms[3] = {sms, room2, room4};
     int best = 0;
     for (int i = 1; i < 3; i++)
@@ -562,29 +548,39 @@ static int choose_split(int M, int K, int T, int sms, int room2, int room4) {
     return 1 << best;
 }
 
+// Eight stages instead of four where a tile has one CTA, if they fit: where a row is long and its weights serve several column
+// tiles, which then come from L2 (28672 x 4096 x 512 727 us with four, 684 with eight; 128256 x 4096 x 32 208, 200; 4096 x 4096
+// x 1500 313, 293), and for small matrices (9728 x 896 x 9 6.9, 6.5; x 1500 197, 195).  Four where a matrix streams once (65536 x 2048 x 9
+// 36.6, 38.7) or is large with rows so short that the ring runs into the next tile (65536 x 896 x 128 113.6, 116.1).  Shared
+// tiles take six (4096 x 14336 x 24: 35.0, 33.8, 34.2 with four, six, eight).
+static bool deep_ring(int M, int K, int T) {
+    const bool small = (long)M * K <= (T > 16 ? 16L : 10L) << 20;
+    return (small || (T > 16 && K >= 2048)) && smem_bytes<16, 4, 8, 1, 8>(K / 32) <= MAX_SMEM;
+}
+
 // CTAs (S = 1) or clusters of S CTAs that the current device holds at once, asked for once per device
-template <int NT, int CB, int EW, int S>
+template <int NT, int CB, int EW, int S, int NST>
 static int room() {
     static std::atomic<int> known[64];
     int dev = 0;
     if (S == 1 || cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return sm_count() / S;
     int n = known[dev].load(std::memory_order_relaxed);
     if (n > 0) return n;
-    if (cudaFuncSetAttribute(k_q8_gemm_tc<NT, CB, EW, S>, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024) != cudaSuccess) {
+    if (cudaFuncSetAttribute(k_q8_gemm_tc<NT, CB, EW, S, NST>, cudaFuncAttributeMaxDynamicSharedMemorySize, MAX_SMEM) != cudaSuccess) {
         cudaGetLastError();
         return 0;
     }
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)(sm_count() / S * S));
-    cfg.blockDim = dim3(Cfg<NT, CB, EW, S>::THREADS);
-    cfg.dynamicSmemBytes = 220 * 1024;
+    cfg.blockDim = dim3(Cfg<NT, CB, EW, S, NST>::THREADS);
+    cfg.dynamicSmemBytes = MAX_SMEM;
     cudaLaunchAttribute at[1];
     at[0].id = cudaLaunchAttributeClusterDimension;
     at[0].val.clusterDim.x = S;
     at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
     cfg.attrs = at;
     cfg.numAttrs = 1;
-    if (cudaOccupancyMaxActiveClusters(&n, k_q8_gemm_tc<NT, CB, EW, S>, &cfg) != cudaSuccess) {
+    if (cudaOccupancyMaxActiveClusters(&n, k_q8_gemm_tc<NT, CB, EW, S, NST>, &cfg) != cudaSuccess) {
         cudaGetLastError();
         return 0;
     }
@@ -592,36 +588,31 @@ static int room() {
     return n;
 }
 
-template <int NT, int CB, int EW, int S>
+template <int NT, int CB, int EW, int S, int NST>
 static int launch(const int8_t* Wq, const uint16_t* Wd, const int8_t* Xq, const uint16_t* Xd, const float* Resid,
                   int resid_ld, float* Y, int M, int K, int T, cudaStream_t s) {
-    using C = Cfg<NT, CB, EW, S>;
+    using C = Cfg<NT, CB, EW, S, NST>;
     const int nb = K / 32;
     CUtensorMap tmW, tmX;
     int rc = make_map(&tmW, Wq, M, K, CB * 32, TM);
     if (rc != LT_OK) return rc;
     rc = make_map(&tmX, Xq, T, K, CB * 32, NT);
     if (rc != LT_OK) return rc;
-    // as many stages as fit: a chunk of 18 KB is on its way for a microsecond or two (4 stages -> 8: 28672 x 4096 x 512
-    // 727 -> 684 us, 128256 x 4096 x 32 210 -> 204, narrow batches within 6 % either way)
-    const size_t rest = 1024 + 1024 + C::XCHG + (size_t)nb * NT * 4;
-    int nstage = C::NSTAGE_MIN;
-    while (nstage < 8 && rest + (size_t)(nstage + 2) * C::STAGE <= 220 * 1024) nstage += 2;
-    const size_t smem = rest + (size_t)nstage * C::STAGE;
-    LT_REQUIRE(smem <= 220 * 1024, "lt_q8_gemm_tc: K=%d needs %zu bytes of shared memory per CTA", K, smem);
+    const size_t smem = smem_bytes<NT, CB, EW, S, NST>(nb);
+    LT_REQUIRE(smem <= MAX_SMEM, "lt_q8_gemm_tc: K=%d needs %zu bytes of shared memory per CTA", K, smem);
     static PerDeviceOnce attr_once;
     if (attr_once.first()) {
-        LT_CUDA(cudaFuncSetAttribute(k_q8_gemm_tc<NT, CB, EW, S>, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024));
+        LT_CUDA(cudaFuncSetAttribute(k_q8_gemm_tc<NT, CB, EW, S, NST>, cudaFuncAttributeMaxDynamicSharedMemorySize, MAX_SMEM));
     }
     Params P;
     P.Wd = (const __half*)Wd; P.Xd = (const __half*)Xd; P.Resid = Resid; P.Y = Y;
     P.status = device_status_ptr();
     LT_REQUIRE(P.status != nullptr, "lt_q8_gemm_tc: status word unavailable");
-    P.M = M; P.K = K; P.T = T; P.resid_ld = resid_ld; P.nstage = nstage;
+    P.M = M; P.K = K; P.T = T; P.resid_ld = resid_ld;
     P.row_tiles = (M + TM - 1) / TM;
     P.t_tiles = (T + NT - 1) / NT;
     const long tiles = (long)P.row_tiles * P.t_tiles;
-    const int most = room<NT, CB, EW, S>();
+    const int most = room<NT, CB, EW, S, NST>();
     LT_REQUIRE(most > 0, "lt_q8_gemm_tc: this device has no room for clusters of %d", S);
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)((tiles < most ? tiles : most) * S));
@@ -636,7 +627,7 @@ static int launch(const int8_t* Wq, const uint16_t* Wd, const int8_t* Xq, const 
         cfg.attrs = at;
         cfg.numAttrs = 1;
     }
-    return check_launch("lt_q8_gemm_tc", 1, cudaLaunchKernelEx(&cfg, k_q8_gemm_tc<NT, CB, EW, S>, tmW, tmX, P));
+    return check_launch("lt_q8_gemm_tc", 1, cudaLaunchKernelEx(&cfg, k_q8_gemm_tc<NT, CB, EW, S, NST>, tmW, tmX, P));
 }
 
 }  // namespace tc
@@ -656,14 +647,15 @@ extern "C" int lt_q8_gemm_tc(const int8_t* Wq, const uint16_t* Wd, const int8_t*
                "lt_q8_gemm_tc: Y may alias Resid only when Resid has one row per column");
     cudaStream_t s = (cudaStream_t)stream;
     if (variant == 0) {
-        const int S = tc::choose_split(M, K, T, tc::sm_count(), tc::room<16, 4, 8, 2>(), tc::room<16, 4, 8, 4>());
+        const int S = tc::choose_split(M, K, T, sm_count(), tc::room<16, 4, 8, 2, 6>(), tc::room<16, 4, 8, 4, 6>());
         variant = S == 4 ? 5 : (S == 2 ? 4 : 1);
     }
-    if (variant == 1) return tc::launch<16, 4, 8, 1>(Wq, Wd, Xq, Xd, Resid, resid_ld, Y, M, K, T, s);
-    if (variant == 2) return tc::launch<32, 1, 8, 1>(Wq, Wd, Xq, Xd, Resid, resid_ld, Y, M, K, T, s);
-    if (variant == 3) return tc::launch<16, 4, 16, 1>(Wq, Wd, Xq, Xd, Resid, resid_ld, Y, M, K, T, s);
-    if (variant == 4) return tc::launch<16, 4, 8, 2>(Wq, Wd, Xq, Xd, Resid, resid_ld, Y, M, K, T, s);
-    if (variant == 5) return tc::launch<16, 4, 8, 4>(Wq, Wd, Xq, Xd, Resid, resid_ld, Y, M, K, T, s);
+    if (variant == 1 && tc::deep_ring(M, K, T)) return tc::launch<16, 4, 8, 1, 8>(Wq, Wd, Xq, Xd, Resid, resid_ld, Y, M, K, T, s);
+    if (variant == 1) return tc::launch<16, 4, 8, 1, 4>(Wq, Wd, Xq, Xd, Resid, resid_ld, Y, M, K, T, s);
+    if (variant == 2) return tc::launch<32, 1, 8, 1, 8>(Wq, Wd, Xq, Xd, Resid, resid_ld, Y, M, K, T, s);
+    if (variant == 3) return tc::launch<16, 4, 16, 1, 4>(Wq, Wd, Xq, Xd, Resid, resid_ld, Y, M, K, T, s);
+    if (variant == 4) return tc::launch<16, 4, 8, 2, 6>(Wq, Wd, Xq, Xd, Resid, resid_ld, Y, M, K, T, s);
+    if (variant == 5) return tc::launch<16, 4, 8, 4, 6>(Wq, Wd, Xq, Xd, Resid, resid_ld, Y, M, K, T, s);
     set_error("lt_q8_gemm_tc: unknown variant %d", variant);
     return LT_ERR_INVALID;
 }
