@@ -512,12 +512,13 @@ static int launch_attn_prefill_wide(const float* Q, int q_ld, const float* K, co
 // independent, so both are halves of a blocked fp32 product whose inner loop runs in the declared order.  What the
 // 16-row form above spends its time on is operand reads (6 of 16 bytes per 32 multiply-adds, 256 of 512 threads
 // folding, one CTA per SM, phases between barriers).  Here a thread owns 4 rows x 4 positions, then 4 rows x HD / 16
-// elements: 8 reads, 4 of them nearly broadcasts, per 64 multiply-adds, and four CTAs overlap on an SM.  Scores are
-// computed twice, first for the row maxima alone: no SM holds 32 rows of scores beside the tiles, and nothing depends
-// on Lmax.  A row's 64 softmax lanes are the 64 positions of a tile, so the lane sums of the denominator stay in the
-// registers of the threads that make the probabilities.  Bound by the multiply-adds (three products of Lmax^2 / 2 x
-// HD per head) and by the uneven lengths of the rows.
-// 2048 positions: 14 heads on 2 of 64: 505 us with 16 rows, now 350; 32 heads on 8 of 128: 3273, now 1549.
+// elements: 8 reads, 4 of them nearly broadcasts, per 64 multiply-adds, and CTAs overlap on an SM (four with heads of 64,
+// two with heads of 128: 52 and 93 KB of shared memory).  Scores are computed twice, first for the row maxima alone: no SM
+// holds 32 rows of scores beside the tiles, and nothing depends on Lmax.  A row's 64 softmax lanes are the 64 positions of
+// a tile, so the lane sums of the denominator stay in the registers of the threads that make the probabilities.  Bound by the operand reads and the multiply-adds together (three
+// products of Lmax^2 / 2 x HD per head, 45 % of the multiply-adds' rate at 2048 positions) and by the uneven lengths of
+// the rows.
+// 2048 positions: 14 heads on 2 of 64: 505 us with 16 rows, now 347; 32 heads on 8 of 128: 3273, now 1549.
 // (64 rows per CTA, 8 x 4 per thread: 444; the 448 CTAs are all resident at once and share the SMs unevenly.)
 constexpr int PB_TILE = 64;
 
@@ -777,9 +778,11 @@ template <int HD>
 static int pick_attn_prefill(const float* Q, int q_ld, const float* K, const float* V, const int* len, float* OUT,
                              int out_ld, int nh, int nkv, float scale, int nrows, int maxt, cudaStream_t s) {
     if (nrows >= 32 && aligned16(V)) {
-        // 32 rows per CTA from three CTAs per SM on: 1000 rows of 14 heads (448 CTAs) take 147 us either way; below,
-        // smaller tiles fill the SMs better (333 rows: 31 us with 16 rows per CTA, 39 with 32) ...
-        if ((long)((nrows + 31) / 32) * nh >= 448)
+        // 32 rows per CTA from three CTAs for each SM on; below, smaller tiles fill the SMs better.  Heads of 64, 14 of them:
+        // 333 rows (154 CTAs) 28 us with 16 rows per CTA, 37 with 32, 850 rows (378) 112 either way, 1200 rows (532) 196 and 183.
+        // Heads of 128 cross between 320 and 450 CTAs: 16 heads, 600 rows (304) 118 and 122, 700 rows (352) 151 and 139;
+        // 32 heads behind 700 positions, 400 rows (416) 359 and 376, 448 rows (448) 404 and 389 ...
+        if ((long)((nrows + 31) / 32) * nh >= 3L * sm_count())
             return launch_attn_prefill_block<HD, 32>(Q, q_ld, K, V, len, OUT, out_ld, nh, nkv, scale, nrows, maxt, s);
         // ... where the score rows of 16 queries fit one SM beside double-buffered tiles
         if (attn_prefill_wide_smem<HD>(maxt) <= 227 * 1024)

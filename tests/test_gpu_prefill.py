@@ -193,3 +193,23 @@ def test_attention_of_long_chunks_equals_one_token_attention(hd, nh, nkv, L0, T)
                   one.data_ptr(), hd, nh, nkv, scale, maxseq, stream())
         assert np.array_equal(bits(got[r]), bits(host(one))), r
     assert _lib.device_status() == set()
+
+
+@pytest.mark.parametrize("hd,nh,nkv,T", [(64, 14, 2, 993), (128, 32, 8, 449), (64, 14, 2, 100)])
+def test_attention_with_v_off_the_16_byte_grid(hd, nh, nkv, T):
+    """The kernels that copy V by 16 bytes are not taken; the result has the same bits."""
+    g = torch.Generator(device="cuda").manual_seed(T)
+    Q, K = torch.randn(T, nh * hd, generator=g, device="cuda"), torch.randn(T, nkv * hd, generator=g, device="cuda")
+    V = torch.randn(T * nkv * hd, generator=g, device="cuda")
+    off = torch.zeros(len(V) + 4, device="cuda")[2:2 + len(V)]
+    off.copy_(V)
+    assert off.data_ptr() % 16 == 8
+    ln = torch.tensor([T], dtype=torch.int32, device="cuda")
+    out = []
+    for v in (V, off):
+        o = torch.full((T, nh * hd), float("nan"), device="cuda")
+        _lib.call("lt_attn_prefill", Q.data_ptr(), nh * hd, K.data_ptr(), v.data_ptr(), ln.data_ptr(), o.data_ptr(), nh * hd, hd, nh, nkv,
+                  float(np.float32(hd ** -0.5)), T, T, stream())
+        out.append(bits(host(o)))
+    assert np.array_equal(*out)
+    assert _lib.device_status() == set()
