@@ -837,7 +837,8 @@ __device__ __forceinline__ void attention_layer(const lt_decode_desc& P, const l
     // Cached V rows are staged in shared memory.  A context with more rows than fit goes through it in segments of seg
     // rows, four buffers: the first four now, the others during the V fold, each when the one four before it is folded
     // (warps 3.. copy, warps 0 and 1 fold).  Folding the rest from global memory, eight rows per round trip to L2, cost
-    // more than the whole rest of the layer: 1000 positions 1178 us per token, now 811 us (32 positions: 380).
+    // more than the whole rest of the layer: 1000 positions 1178 us per token, 811 in segments, and 708 with the K rows by whole
+    // sectors below (32 positions: 380).
     const int seg = vcap / 16 * 4;
     const bool in_segments = Lc > vcap && seg > 0;
     const int nseg = in_segments ? (Lc + seg - 1) / seg : 0;
@@ -945,7 +946,7 @@ __device__ __forceinline__ void attention_layer(const lt_decode_desc& P, const l
         if (hf == 1 && t < L) A.sh[t] = __fmul_rn(s, P.scale);
     }
     // contexts longer than the registers hold: a thread per position, half a row on its way at once, by whole sectors
-    // (16-byte loads of 32 different rows fetch every sector twice: the carve-out leaves no L1 to keep the other half).  1000 positions: 811 -> 708 us per token
+    // (16-byte loads of 32 different rows fetch every sector twice: the carve-out leaves no L1 to keep the other half).  1000 positions: 811 us per token, now 708
     for (int t = tid + KPOS; t < L; t += DEC_CTHREADS) {
         const float4* q4 = (const float4*)A.q;
         float s = 0.0f;

@@ -1,6 +1,8 @@
 """GPU: the device-resident decode engine (forward_pass_resident / GraphRunner, the
 reference's entry points) against the CPU oracle engine, plus the reference's own
 graph-replay == eager contract (bit-exact logits, tokens, device length, cache rows)."""
+import ctypes
+
 import numpy as np
 import pytest
 import torch
@@ -343,6 +345,39 @@ def test_one_kernel_step_in_long_contexts_equals_per_op_graph(context):
         finally:
             dr._FUSED_STEP = old
             dr.apply_production_profile()
+    for i, (a, b) in enumerate(zip(*out)):
+        assert np.array_equal(a, b), i
+    assert dr._lib.device_status() == set()
+
+
+@pytest.mark.parametrize("arch,context,shift,kw", [("tiny", 300, 0, {}), ("tiny", 2100, 0, {}), ("qwen2.5-0.5b", 600, 4, dict(n_layers=2)),
+                                                   ("tiny", 310, 4, {})])
+def test_one_kernel_step_of_small_heads_and_off_grid_caches_equals_per_op_graph(arch, context, shift, kw, monkeypatch):
+    """Long contexts with heads of 32 (2100 positions: more V rows than an attention CTA stages), and caches that start 16 bytes
+    off the 32-byte grid, whose K rows are read by 16 bytes."""
+    if shift:
+        make = dr.DeviceKVCache.__init__
+
+        def shifted(self, max_seq, nkv, hd, elem_bytes=4):
+            make(self, max_seq, nkv, hd, elem_bytes)
+            self._k, self._v = (torch.zeros(len(t) + 8, device="cuda")[shift:shift + len(t)] for t in (self._k, self._v))
+            self.k_ptr, self.v_ptr = ctypes.c_void_p(self._k.data_ptr()), ctypes.c_void_p(self._v.data_ptr())
+            assert self._k.data_ptr() % 32 == 16
+        monkeypatch.setattr(dr.DeviceKVCache, "__init__", shifted)
+    out = []
+    for mode in ("persistent", False):
+        m, w, cfg = _fresh(arch, seed=3, **kw)
+        toks = _prompt(m["cfg"]["vocab"], context + 4, seed=context)
+        dr._KV_MAX_SEQ = context + 16
+        monkeypatch.setattr(dr, "_FUSED_STEP", mode)
+        kv = [None] * cfg["n_layers"]
+        gr = dr.GraphRunner(w, cfg, kv)
+        gr.seed(torch.tensor(toks[:context]), torch.arange(context))
+        gr.capture(torch.tensor([toks[context]]), torch.tensor([context]))
+        if mode == "persistent":
+            assert gr.launches_per_token == 1
+        out.append([bits(gr.replay_logits(t).reshape(-1).numpy()).copy() for t in toks[context:]])
+    dr.apply_production_profile()
     for i, (a, b) in enumerate(zip(*out)):
         assert np.array_equal(a, b), i
     assert dr._lib.device_status() == set()
