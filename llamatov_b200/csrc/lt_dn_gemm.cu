@@ -286,7 +286,8 @@ static int launch_tc(const void* W, int ldw, const void* X, int ldx, GemmP P, cu
 
 // ---------------------------------------------------------------------------- fp32
 
-// ---- fp32: every product and sum an fp32 fused multiply-add on the CUDA cores, which bound it.  64 weight rows x 8 MQ
+// ---- fp32: every product and sum an fp32 fused multiply-add on the CUDA cores, bound by the operand reads (shared memory 76
+// to 79 % busy, issue slots 70 %, FMA pipe 48 %).  64 weight rows x 8 MQ
 // tokens per CTA of 128 threads, a thread owns 4 rows (pairs of rows with GLU) x MQ tokens: 4 + MQ 16-byte reads of shared
 // memory per 16 MQ multiply-adds, three stages of 32 k filled by asynchronous copies.  k is summed in up to four contiguous
 // parts, added in order.  One CTA folds them in turn, or a cluster of as many CTAs takes one each and adds them through

@@ -515,9 +515,9 @@ static int launch_attn_prefill_wide(const float* Q, int q_ld, const float* K, co
 // elements: 8 reads, 4 of them nearly broadcasts, per 64 multiply-adds, and CTAs overlap on an SM (four with heads of 64,
 // two with heads of 128: 52 and 93 KB of shared memory).  Scores are computed twice, first for the row maxima alone: no SM
 // holds 32 rows of scores beside the tiles, and nothing depends on Lmax.  A row's 64 softmax lanes are the 64 positions of
-// a tile, so the lane sums of the denominator stay in the registers of the threads that make the probabilities.  Bound by the operand reads and the multiply-adds together (three
-// products of Lmax^2 / 2 x HD per head, 45 % of the multiply-adds' rate at 2048 positions) and by the uneven lengths of
-// the rows.
+// a tile, so the lane sums of the denominator stay in the registers of the threads that make the probabilities.  Bound by the operand reads and issue slots of its three
+// products of Lmax^2 / 2 x HD per head (2048 positions: shared memory 74 % busy, issue slots 70 %, FMA pipe 49 %) and by the
+// uneven lengths of the rows.
 // 2048 positions: 14 heads on 2 of 64: 505 us with 16 rows, now 347; 32 heads on 8 of 128: 3273, now 1549.
 // (64 rows per CTA, 8 x 4 per thread: 444; the 448 CTAs are all resident at once and share the SMs unevenly.)
 constexpr int PB_TILE = 64;
