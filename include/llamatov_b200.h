@@ -94,11 +94,11 @@ int lt_q8_gemv(const int8_t* Wq, const uint16_t* Wd, const int8_t* Xq, const uin
  * fp32 scale-and-fold runs in the frozen order on the CUDA cores.  This is the batched form the
  * reference does not have (its prefill loops the per-token GEMV and requires batched results to
  * equal the per-token ones, bpd/lib/dev_residency.py:1344-1350).  K must be a multiple of 128.
- * variant: 0 = default: form 1, where few tiles would leave SMs idle with clusters of two or four CTAs that share a
- * tile's blocks; 1 = 16-column tiles, 128-byte weight chunks, 8 epilogue warps (the matrix
- * streams once from HBM in 128-byte rows; fastest measured at every width); 2 = 32-column tiles,
+ * variant: 0 = default: form 6 where it is the faster one, else form 1, where few tiles would leave SMs idle with clusters of
+ * two or four CTAs that share a tile's blocks; 1 = 16-column tiles, 128-byte weight chunks, 8 epilogue warps (the matrix
+ * streams once from HBM in 128-byte rows); 2 = 32-column tiles,
  * 32-byte chunks (fewest live partials per thread); 3 = as 1 with 16 epilogue warps; 4, 5 = form 1 with clusters of two,
- * four CTAs.
+ * four CTAs; 6 = 32-column tiles whose products of scales come from the tensor cores too, without a limit on K.
  * Resid: NULL, or a bias of M entries added to every column (resid_ld = 0), or one row per
  * column, Resid[t * resid_ld + n] (the residual stream of a prefill; Y may then alias Resid).
  * lt_q8_gemv forwards to this entry for T > 8 when K allows it. */
@@ -108,6 +108,8 @@ int lt_q8_gemm_tc(const int8_t* Wq, const uint16_t* Wd, const int8_t* Xq, const 
 /* How many CTAs (1, 2 or 4) the default form has share a tile on a GPU with sms SMs that holds clusters2 and clusters4
  * clusters of two and four CTAs at once; 0 for sizes that the entry above refuses.  Host arithmetic, no GPU needed. */
 int lt_q8_gemm_tc_split(int M, int K, int T, int sms, int clusters2, int clusters4);
+/* Whether the default is form 6 there.  Host arithmetic, no GPU needed. */
+int lt_q8_gemm_tc_pair(int M, int K, int T, int sms, int clusters2, int clusters4);
 
 /* ---- RMSNorm --------------------------------------------------------------------------
  * replaces k_rmsnorm, mode block_row (bpd/kernelgen/emitters/norm_softmax_from_facts.pl:83-108;

@@ -81,6 +81,7 @@ _RESTYPES = {"lt_last_error": ctypes.c_char_p, "lt_version": ctypes.c_char_p,
              "lt_launch_count": ctypes.c_ulonglong}
 # name -> (argtypes, restype) for the entries that return something other than a status code
 _QUERIES = {"lt_q8_gemm_tc_split": ([_i, _i, _i, _i, _i, _i], ctypes.c_int),
+            "lt_q8_gemm_tc_pair": ([_i, _i, _i, _i, _i, _i], ctypes.c_int),
             "lt_attn_decode_batch_scratch_floats": ([_i, _i, _i], ctypes.c_long),
             "lt_attn_decode_split_scratch_floats": ([_i, _i, _i, _i], ctypes.c_long),
             "lt_set_chained_launch": ([_i], ctypes.c_int)}
