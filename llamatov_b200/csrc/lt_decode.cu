@@ -757,11 +757,9 @@ __device__ __forceinline__ void norm_quant(const float* sF, const float* sW, int
         for (int k = 0; k < 2; k++) {
             const int bb = b0 + k * DEC_CWARPS;
             if (bb < nblk) {
-                const float d = (m[k] > 0.0f) ? __fdiv_rn(m[k], 127.0f) : 1.0f;
-                const __half dh = __float2half_rn(d);
-                int q = (int)rintf(__fdiv_rn(v[k], __half2float(dh)));
-                q = q < -127 ? -127 : (q > 127 ? 127 : q);
-                sXq[bb * 32 + lane] = (int8_t)q;
+                const __half dh = q8_scale(m[k]);
+                const float dq = __half2float(dh);
+                sXq[bb * 32 + lane] = (int8_t)q8_value(v[k], dq, q8_reciprocal(dq));
                 if (lane == 0) sXd[bb] = dh;
             }
         }

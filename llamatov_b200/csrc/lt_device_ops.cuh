@@ -33,12 +33,22 @@ __device__ __forceinline__ void rope_pair(float x1, float x2, int j, int hd, flo
 }
 
 // ---- RMSNorm and quantiser over a vector in shared memory, for kernels that fuse them as a prologue
-// sum of squares in the declared 256-lane order; the block has exactly 256 threads
+// sum of squares in the declared 256-lane order; blocks of at least 256 threads
 __device__ __forceinline__ float block_rms_sumsq(const float* sF, int N, float* sred) {
     const int t = threadIdx.x;
     float local = 0.0f;
-    if (t < 256)
-        for (int j = t; j < N; j += 256) local = __fmaf_rn(sF[j], sF[j], local);
+    if (t < 256) {
+        int j = t;
+#pragma unroll 1
+        for (; j + 768 < N; j += 1024) {    // four reads on their way per step of the chain
+            const float a = sF[j], b = sF[j + 256], c = sF[j + 512], d = sF[j + 768];
+            local = __fmaf_rn(a, a, local);
+            local = __fmaf_rn(b, b, local);
+            local = __fmaf_rn(c, c, local);
+            local = __fmaf_rn(d, d, local);
+        }
+        for (; j < N; j += 256) local = __fmaf_rn(sF[j], sF[j], local);
+    }
     if (t < 256) sred[t] = local;
     __syncthreads();
     if (t < 32) {
@@ -52,33 +62,30 @@ __device__ __forceinline__ float block_rms_sumsq(const float* sF, int N, float* 
     return sred[256];
 }
 
-// quantise N floats of shared memory (optionally (x*inv)*w first) into sXq / sXd; all warps
+// quantise N floats of shared memory (optionally (x*inv)*w first) into sXq / sXd; all warps.  Eight threads per block, four values
+// each (16-byte aligned vectors).  A lane per value with divisions took three times the instructions, which the CTAs of an SM
+// share: a GEMV of 6144 x 4096 behind a norm 12.7 us, now 10.3 (7.2 without the norm).
 __device__ __forceinline__ void block_quant(const float* sF, const float* sW, float inv, int N, int8_t* sXq,
                                             __half* sXd) {
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
-    const int nblk = N >> 5;
-    for (int b0 = warp; b0 < nblk; b0 += 2 * nw) {
-        float v[2], a[2];
-#pragma unroll
-        for (int k = 0; k < 2; k++) {
-            const int b = b0 + k * nw;
-            const int j = (b < nblk ? b : b0) * 32 + lane;
-            float x = sF[j];
-            if (sW != nullptr) x = __fmul_rn(__fmul_rn(x, inv), sW[j]);
-            v[k] = x;
-            a[k] = __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(fabsf(x))));
+    const int nquad = N >> 2;      // a multiple of 8: the eight threads of a block are in or out together
+    for (int i0 = threadIdx.x & ~31; i0 < nquad; i0 += blockDim.x) {
+        const int i = i0 + (threadIdx.x & 31);
+        float4 x = i < nquad ? ((const float4*)sF)[i] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        if (sW != nullptr && i < nquad) {
+            const float4 w = ((const float4*)sW)[i];
+            x.x = __fmul_rn(__fmul_rn(x.x, inv), w.x); x.y = __fmul_rn(__fmul_rn(x.y, inv), w.y);
+            x.z = __fmul_rn(__fmul_rn(x.z, inv), w.z); x.w = __fmul_rn(__fmul_rn(x.w, inv), w.w);
         }
+        unsigned m = max(max(__float_as_uint(fabsf(x.x)), __float_as_uint(fabsf(x.y))),
+                         max(__float_as_uint(fabsf(x.z)), __float_as_uint(fabsf(x.w))));
 #pragma unroll
-        for (int k = 0; k < 2; k++) {
-            const int b = b0 + k * nw;
-            if (b < nblk) {
-                const float d = (a[k] > 0.0f) ? __fdiv_rn(a[k], 127.0f) : 1.0f;
-                const __half dh = __float2half_rn(d);
-                int q = (int)rintf(__fdiv_rn(v[k], __half2float(dh)));
-                q = q < -127 ? -127 : (q > 127 ? 127 : q);
-                sXq[b * 32 + lane] = (int8_t)q;
-                if (lane == 0) sXd[b] = dh;
-            }
+        for (int s = 4; s > 0; s >>= 1) m = max(m, __shfl_xor_sync(0xffffffffu, m, s));
+        const __half dh = q8_scale(__uint_as_float(m));
+        const float dq = __half2float(dh), r = q8_reciprocal(dq);
+        const int q0 = q8_value(x.x, dq, r), q1 = q8_value(x.y, dq, r), q2 = q8_value(x.z, dq, r), q3 = q8_value(x.w, dq, r);
+        if (i < nquad) {
+            ((char4*)sXq)[i] = make_char4((signed char)q0, (signed char)q1, (signed char)q2, (signed char)q3);
+            if ((i & 7) == 0) sXd[i >> 3] = dh;
         }
     }
 }

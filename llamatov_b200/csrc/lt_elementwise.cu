@@ -9,8 +9,8 @@ namespace lt {
 
 // ------------------------------------------------------------------ quantiser
 // Four elements per thread: bound by the bytes (5 per element) once there are enough of them; a warp per block, one
-// element per lane (k_quant_q8_lane), issues four times the loads and stores and twice the divisions
-// (2048 x 4864: 29.6 us, 18.5 with four; 2048 x 896: 8.3, 5.3).
+// element per lane (k_quant_q8_lane), issues four times the loads and stores and works on a scale in every lane
+// (2048 x 4864: 22.8 us, 10.1 with four; 2048 x 896: 5.5, 3.1).
 __global__ void __launch_bounds__(256) k_quant_q8(const float* __restrict__ X, int8_t* __restrict__ Xq,
                                                   __half* __restrict__ Xd, long nblocks) {
     const long i = (long)blockIdx.x * 256 + threadIdx.x;      // quad of elements
@@ -25,8 +25,8 @@ __global__ void __launch_bounds__(256) k_quant_q8(const float* __restrict__ X, i
     ((char4*)Xq)[i] = q;
 }
 
-// One warp per 32-block, lane = element; any alignment.  Its chain of divisions is a quarter as long, which counts while every
-// block has a resident warp of its own (1 x 4864: 1.47 us, 1.53 with four elements per thread; 300 x 896: 1.70, 2.00).
+// One warp per 32-block, lane = element; any alignment.  Its chain is a quarter as long, which counts while every block has a
+// resident warp of its own (300 x 896: 1.79 us, 1.83 with four elements per thread; 400 x 896: 2.21, 1.91).
 __global__ void __launch_bounds__(256) k_quant_q8_lane(const float* __restrict__ X, int8_t* __restrict__ Xq,
                                                    __half* __restrict__ Xd, long nblocks) {
     long b = (long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
