@@ -291,6 +291,24 @@ int lt_silu_mul_quant_rows(const float* g, const float* u, int ld, int8_t* Xq, u
 int lt_attn_prefill(const float* Q, int q_ld, const float* K, const float* V, const int* len, float* OUT,
                     int out_ld, int hd, int nh, int nkv, float scale, int nrows, int maxt, void* stream);
 
+/* Chunks of T new rows of up to LT_ROW_SEQS sequences, one after the other in the rows of a matrix: each has caches of k and v rows
+ * (nkv * hd floats, room for max_seq), a device length, and start rows before the chunk. */
+#define LT_ROW_SEQS 8
+typedef struct {
+    float* k[LT_ROW_SEQS];
+    float* v[LT_ROW_SEQS];
+    int* len[LT_ROW_SEQS];
+    int start[LT_ROW_SEQS];
+    int max_seq[LT_ROW_SEQS];
+} lt_row_seqs;
+/* lt_rope_rows of the q and k heads and lt_append_kv_rows with the increment, for all of them in one launch: row b * T + r of X (nh
+ * q heads, nkv k heads, nkv v heads of hd at the row start, row stride ld) is at position start[b] + r; len[b] becomes start[b] + T. */
+int lt_rope_append_rows(float* X, int ld, const lt_row_seqs* seqs, int B, int T, int nh, int nkv, int hd, float theta, void* stream);
+/* lt_attn_prefill of all of them (the same bits), after lt_rope_append_rows. */
+int lt_attn_prefill_rows(const float* Q, int q_ld, const lt_row_seqs* seqs, int B, int T, float* OUT, int out_ld, int hd, int nh,
+                         int nkv, float scale, void* stream);
+
+
 /* ---- decode operators for a batch of sequences / long contexts ------------------------------
  * No batched engine exists in the reference; its contract is that every sequence gets the
  * one-sequence result.  The KV caches of a batch are one buffer per layer,

@@ -54,6 +54,8 @@ SIGNATURES = {
     "lt_rope_rows": [_vp, _i, _vp, _i, _i, _i, _f, _vp],
     "lt_append_kv_rows": [_vp, _vp, _vp, _vp, _i, _vp, _i, _i, _i, _i, _vp],
     "lt_silu_mul_quant_rows": [_vp, _vp, _i, _vp, _vp, _i, _i, _vp],
+    "lt_rope_append_rows": [_vp, _i, _vp, _i, _i, _i, _i, _i, _f, _vp],
+    "lt_attn_prefill_rows": [_vp, _i, _vp, _i, _i, _vp, _i, _i, _i, _i, _f, _vp],
     "lt_attn_prefill": [_vp, _i, _vp, _vp, _vp, _vp, _i, _i, _i, _i, _f, _i, _i, _vp],
     "lt_rope_batch": [_vp, _i, _vp, _i, _i, _i, _f, _vp],
     "lt_append_kv_batch": [_vp, _vp, _vp, _vp, _i, _vp, _i, _i, _i, _i, _vp],
@@ -85,6 +87,14 @@ _QUERIES = {"lt_q8_gemm_tc_split": ([_i, _i, _i, _i, _i, _i], ctypes.c_int),
             "lt_attn_decode_batch_scratch_floats": ([_i, _i, _i], ctypes.c_long),
             "lt_attn_decode_split_scratch_floats": ([_i, _i, _i, _i], ctypes.c_long),
             "lt_set_chained_launch": ([_i], ctypes.c_int)}
+
+
+ROW_SEQS = 8
+
+
+class RowSeqs(ctypes.Structure):
+    """lt_row_seqs: the sequences of a launch over rows."""
+    _fields_ = [("k", _vp * ROW_SEQS), ("v", _vp * ROW_SEQS), ("len", _vp * ROW_SEQS), ("start", _i * ROW_SEQS), ("max_seq", _i * ROW_SEQS)]
 
 
 # ---- include/llamatov_b200_dense.h

@@ -51,6 +51,39 @@ __global__ void k_rope_rows(float* __restrict__ X, int ld, const int* __restrict
     X[base + j + half] = o2;
 }
 
+// ------------------------------------------------------------------ rope + KV append of several sequences
+// Rows b * T + r of X (q heads, k heads, v heads of hd) are rotated at position start[b] + r, k and v go to the caches' rows from
+// start[b] on, the lengths become start[b] + T.  A thread has one pair of every head of its part of a row, so that the angle
+// (a power, a sine and a cosine: what k_rope_rows spends its time on) is worked out once for all of them.  2048 rows of 14 + 2 + 2
+// heads of 64: 16.4 us in three launches (rotation 11.7), 6.6 here; three sequences of 333 rows 21.5 us in nine, 5.0 here.
+__global__ void __launch_bounds__(256) k_rope_append_rows(float* __restrict__ X, int ld, const __grid_constant__ lt_row_seqs S, int B,
+                                                          int T, int nh, int nkv, int hd, float theta, int per) {
+    const int half = hd / 2, width = nkv * hd;
+    const long gid = (long)blockIdx.x * 256 + threadIdx.x;
+    const int row = (int)(gid / half), j = (int)(gid - (long)row * half);
+    if (row >= B * T) return;
+    const int b = row / T, r = row - b * T, pos = S.start[b] + r;
+    if (r == 0 && j == 0 && blockIdx.y == 0) *S.len[b] = S.start[b] + T;
+    float c, s;
+    rope_trig(j, hd, theta, pos, c, s);
+    const int h1 = min((int)(blockIdx.y + 1) * per, nh + 2 * nkv);
+#pragma unroll 4
+    for (int h = blockIdx.y * per; h < h1; h++) {
+        float* x = X + (long)row * ld + (long)h * hd + j;
+        float a = x[0], e = x[half];
+        if (h < nh + nkv) {
+            rope_rotate(a, e, c, s, a, e);
+            x[0] = a;
+            x[half] = e;
+        }
+        if (h >= nh) {
+            float* o = (h < nh + nkv ? S.k[b] + (long)(h - nh) * hd : S.v[b] + (long)(h - nh - nkv) * hd) + (long)pos * width + j;
+            o[0] = a;
+            o[half] = e;
+        }
+    }
+}
+
 // ------------------------------------------------------------------ KV append rows
 // rows 0..nrows-1 of ksrc / vsrc (row stride src_ld) go to cache positions *len .. *len+nrows-1
 __global__ void k_append_kv_rows(float* __restrict__ kbase, const float* __restrict__ ksrc, float* __restrict__ vbase,
@@ -122,6 +155,15 @@ __global__ void k_silu_mul_quant_rows_lane(const float* __restrict__ G, const fl
 // lanes + tree, left-fold V sum, / Z.
 constexpr int PF_THREADS = 256;
 constexpr int PF_KTILE = 128;            // K rows staged per tile: two threads per position
+
+// The sequences of a launch.  One: its length on the device; several: their lengths after the append, from the host.  Together
+// short prompts fill the SMs with blocks of 32 rows (three of 333: 87 us one after the other with 16 rows, 55 together).
+struct AttnSeqs {
+    const float *k[LT_ROW_SEQS], *v[LT_ROW_SEQS];
+    const int* len;
+    int total[LT_ROW_SEQS];
+    __device__ __forceinline__ int length(int b) const { return len != nullptr ? *len : total[b]; }
+};
 
 template <int HD, int QT>
 __global__ void __launch_bounds__(PF_THREADS, QT <= 8 ? 3 : 1)
@@ -297,9 +339,8 @@ constexpr int PW_TILE = 128;             // positions per staged tile of K or V 
 
 template <int HD>
 __global__ void __launch_bounds__(PW_THREADS, 1)
-k_attn_prefill_wide(const float* __restrict__ Q, int q_ld, const float* __restrict__ K, const float* __restrict__ V,
-                    const int* __restrict__ len_ptr, float* __restrict__ OUT, int out_ld, int nh, int nkv, float scale,
-                    int nrows, int maxt, int* status) {
+k_attn_prefill_wide(const float* __restrict__ Q, int q_ld, const __grid_constant__ AttnSeqs S, float* __restrict__ OUT, int out_ld, int nh,
+                    int nkv, float scale, int nrows, int maxt, int* status) {
     constexpr int QT = PW_QT, KST = HD + 4;
     extern __shared__ __align__(16) float pf_smem[];
     float* qs = pf_smem;                     // [QT][HD]
@@ -311,7 +352,10 @@ k_attn_prefill_wide(const float* __restrict__ Q, int q_ld, const float* __restri
     const int tid = threadIdx.x;
     const int h = blockIdx.y;
     const int r0 = blockIdx.x * QT;
-    const int Lafter = *len_ptr;
+    const int seq = blockIdx.z, Lafter = S.length(seq);
+    const float *K = S.k[seq], *V = S.v[seq];
+    Q += (long)seq * nrows * q_ld;
+    OUT += (long)seq * nrows * out_ld;
     if (Lafter < nrows || Lafter > maxt) {
         if (tid == 0) atomicOr(status, (int)LT_STATUS_BAD_LENGTH);
         return;
@@ -493,8 +537,8 @@ static size_t attn_prefill_wide_smem(int maxt) {
 }
 
 template <int HD>
-static int launch_attn_prefill_wide(const float* Q, int q_ld, const float* K, const float* V, const int* len, float* OUT,
-                                    int out_ld, int nh, int nkv, float scale, int nrows, int maxt, cudaStream_t s) {
+static int launch_attn_prefill_wide(const float* Q, int q_ld, const AttnSeqs& S, int nseq, float* OUT, int out_ld, int nh, int nkv,
+                                    float scale, int nrows, int maxt, cudaStream_t s) {
     int* st = device_status_ptr();
     LT_REQUIRE(st != nullptr, "lt_attn_prefill: status word unavailable");
     const size_t smem = attn_prefill_wide_smem<HD>(maxt);
@@ -502,8 +546,8 @@ static int launch_attn_prefill_wide(const float* Q, int q_ld, const float* K, co
     if (attr_once.first()) {
         LT_CUDA(cudaFuncSetAttribute(k_attn_prefill_wide<HD>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024));
     }
-    dim3 grid((nrows + PW_QT - 1) / PW_QT, nh);
-    k_attn_prefill_wide<HD><<<grid, PW_THREADS, smem, s>>>(Q, q_ld, K, V, len, OUT, out_ld, nh, nkv, scale, nrows, maxt, st);
+    dim3 grid((nrows + PW_QT - 1) / PW_QT, nh, nseq);
+    k_attn_prefill_wide<HD><<<grid, PW_THREADS, smem, s>>>(Q, q_ld, S, OUT, out_ld, nh, nkv, scale, nrows, maxt, st);
     return check_launch("lt_attn_prefill");
 }
 
@@ -532,9 +576,8 @@ struct PrefillBlock {
 
 template <int HD, int QT>
 __global__ void __launch_bounds__(PrefillBlock<HD, QT>::THREADS)
-k_attn_prefill_block(const float* __restrict__ Q, int q_ld, const float* __restrict__ K, const float* __restrict__ V,
-                     const int* __restrict__ len_ptr, float* __restrict__ OUT, int out_ld, int nh, int nkv, float scale,
-                     int nrows, int maxt, int* status) {
+k_attn_prefill_block(const float* __restrict__ Q, int q_ld, const __grid_constant__ AttnSeqs S, int nseq, float* __restrict__ OUT, int out_ld,
+                     int nh, int nkv, float scale, int nrows, int maxt, int* status) {
     using B = PrefillBlock<HD, QT>;
     constexpr int PB_THREADS = B::THREADS, ST = B::ST, PST = B::PST, MQ = QT * 16 / PB_THREADS, ND = HD / 64;
     extern __shared__ __align__(16) float pf_smem[];
@@ -545,8 +588,12 @@ k_attn_prefill_block(const float* __restrict__ Q, int q_ld, const float* __restr
     float* zs = ps + QT * PST;               // [QT]
     const int tid = threadIdx.x, n = tid & 15, m = tid >> 4;
     const int h = blockIdx.x % nh;
-    const int r0 = ((int)gridDim.x / nh - 1 - (int)blockIdx.x / nh) * QT;     // the longest rows first
-    const int Lafter = *len_ptr;
+    const int step = (int)blockIdx.x / nh, seq = step % nseq;
+    const int r0 = ((int)gridDim.x / nh / nseq - 1 - step / nseq) * QT;       // the longest rows first
+    const int Lafter = S.length(seq);
+    const float *K = S.k[seq], *V = S.v[seq];
+    Q += (long)seq * nrows * q_ld;
+    OUT += (long)seq * nrows * out_ld;
     if (Lafter < nrows || Lafter > maxt) {
         if (tid == 0) atomicOr(status, (int)LT_STATUS_BAD_LENGTH);
         return;
@@ -742,8 +789,8 @@ k_attn_prefill_block(const float* __restrict__ Q, int q_ld, const float* __restr
 }
 
 template <int HD, int QT>
-static int launch_attn_prefill_block(const float* Q, int q_ld, const float* K, const float* V, const int* len, float* OUT,
-                                     int out_ld, int nh, int nkv, float scale, int nrows, int maxt, cudaStream_t s) {
+static int launch_attn_prefill_block(const float* Q, int q_ld, const AttnSeqs& S, int nseq, float* OUT, int out_ld, int nh, int nkv,
+                                     float scale, int nrows, int maxt, cudaStream_t s) {
     int* st = device_status_ptr();
     LT_REQUIRE(st != nullptr, "lt_attn_prefill: status word unavailable");
     constexpr int smem = PrefillBlock<HD, QT>::SMEM;
@@ -751,8 +798,8 @@ static int launch_attn_prefill_block(const float* Q, int q_ld, const float* K, c
     if (attr_once.first()) {
         LT_CUDA(cudaFuncSetAttribute(k_attn_prefill_block<HD, QT>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
     }
-    k_attn_prefill_block<HD, QT><<<(nrows + QT - 1) / QT * nh, PrefillBlock<HD, QT>::THREADS, smem, s>>>(Q, q_ld, K, V, len, OUT, out_ld,
-                                                                                                        nh, nkv, scale, nrows, maxt, st);
+    k_attn_prefill_block<HD, QT><<<(nrows + QT - 1) / QT * nh * nseq, PrefillBlock<HD, QT>::THREADS, smem, s>>>(
+        Q, q_ld, S, nseq, OUT, out_ld, nh, nkv, scale, nrows, maxt, st);
     return check_launch("lt_attn_prefill");
 }
 
@@ -774,20 +821,33 @@ static int launch_attn_prefill(const float* Q, int q_ld, const float* K, const f
     return check_launch("lt_attn_prefill");
 }
 
+// The forms that take several sequences at once, LT_ERR_UNSUPPORTED where none fits
 template <int HD>
-static int pick_attn_prefill(const float* Q, int q_ld, const float* K, const float* V, const int* len, float* OUT,
-                             int out_ld, int nh, int nkv, float scale, int nrows, int maxt, cudaStream_t s) {
-    if (nrows >= 32 && aligned16(V)) {
+static int pick_attn_prefill_rows(const float* Q, int q_ld, const AttnSeqs& S, int nseq, float* OUT, int out_ld, int nh, int nkv,
+                                  float scale, int nrows, int maxt, cudaStream_t s) {
+    bool aligned = true;
+    for (int b = 0; b < nseq; b++) aligned = aligned && aligned16(S.v[b]);
+    if (nrows >= 32 && aligned) {
         // 32 rows per CTA from three CTAs for each SM on; below, smaller tiles fill the SMs better.  Heads of 64, 14 of them:
         // 333 rows (154 CTAs) 28 us with 16 rows per CTA, 37 with 32, 850 rows (378) 112 either way, 1200 rows (532) 196 and 183.
         // Heads of 128 cross between 320 and 450 CTAs: 16 heads, 600 rows (304) 118 and 122, 700 rows (352) 151 and 139;
         // 32 heads behind 700 positions, 400 rows (416) 359 and 376, 448 rows (448) 404 and 389 ...
-        if ((long)((nrows + 31) / 32) * nh >= 3L * sm_count())
-            return launch_attn_prefill_block<HD, 32>(Q, q_ld, K, V, len, OUT, out_ld, nh, nkv, scale, nrows, maxt, s);
+        if ((long)((nrows + 31) / 32) * nh * nseq >= 3L * sm_count())
+            return launch_attn_prefill_block<HD, 32>(Q, q_ld, S, nseq, OUT, out_ld, nh, nkv, scale, nrows, maxt, s);
         // ... where the score rows of 16 queries fit one SM beside double-buffered tiles
         if (attn_prefill_wide_smem<HD>(maxt) <= 227 * 1024)
-            return launch_attn_prefill_wide<HD>(Q, q_ld, K, V, len, OUT, out_ld, nh, nkv, scale, nrows, maxt, s);
+            return launch_attn_prefill_wide<HD>(Q, q_ld, S, nseq, OUT, out_ld, nh, nkv, scale, nrows, maxt, s);
     }
+    return LT_ERR_UNSUPPORTED;
+}
+
+template <int HD>
+static int pick_attn_prefill(const float* Q, int q_ld, const float* K, const float* V, const int* len, float* OUT,
+                             int out_ld, int nh, int nkv, float scale, int nrows, int maxt, cudaStream_t s) {
+    AttnSeqs S = {};
+    S.k[0] = K; S.v[0] = V; S.len = len;
+    const int rc = pick_attn_prefill_rows<HD>(Q, q_ld, S, 1, OUT, out_ld, nh, nkv, scale, nrows, maxt, s);
+    if (rc != LT_ERR_UNSUPPORTED) return rc;
     // query rows per tile: 8 while three CTAs of score rows fit an SM (the V sum and the softmax are
     // chains of dependent operations, resident warps hide them), else 4; 16 only for short chunks
     const size_t per_row = (size_t)((maxt + 3) & ~3) + HD + 65;
@@ -822,6 +882,30 @@ extern "C" int lt_rope_rows(float* X, int ld, const int* pos0, int nrows, int n_
     const long total = (long)nrows * n_head * (hd / 2);
     k_rope_rows<<<(unsigned)((total + 255) / 256), 256, 0, (cudaStream_t)stream>>>(X, ld, pos0, nrows, n_head, hd, theta);
     return check_launch("lt_rope_rows");
+}
+
+static int check_seqs(const char* what, const lt_row_seqs* S, int B, int T) {
+    LT_REQUIRE(S != nullptr && B > 0 && B <= LT_ROW_SEQS && T > 0, "%s: B=%d (1 to %d) T=%d", what, B, LT_ROW_SEQS, T);
+    for (int b = 0; b < B; b++) {
+        LT_REQUIRE(S->k[b] && S->v[b] && S->len[b], "%s: null pointer", what);
+        LT_REQUIRE(S->start[b] >= 0 && S->start[b] + (long)T <= S->max_seq[b], "%s: %d + %d positions exceed %d", what, S->start[b], T,
+                   S->max_seq[b]);
+    }
+    return LT_OK;
+}
+
+extern "C" int lt_rope_append_rows(float* X, int ld, const lt_row_seqs* seqs, int B, int T, int nh, int nkv, int hd, float theta,
+                                   void* stream) {
+    const int rc = check_seqs("lt_rope_append_rows", seqs, B, T);
+    if (rc != LT_OK) return rc;
+    LT_REQUIRE(X && nh > 0 && nkv > 0 && hd > 0 && hd % 2 == 0 && ld >= (nh + 2 * nkv) * hd && (long)B * T < (1L << 31),
+               "lt_rope_append_rows: nh=%d nkv=%d hd=%d ld=%d", nh, nkv, hd, ld);
+    const long threads = (long)B * T * (hd / 2);
+    const int heads = nh + 2 * nkv;
+    const int per = threads >= 512L * sm_count() ? heads : (heads + 3) / 4;     // few rows: the heads of a row in four parts
+    dim3 grid((unsigned)((threads + 255) / 256), (unsigned)((heads + per - 1) / per));
+    k_rope_append_rows<<<grid, 256, 0, (cudaStream_t)stream>>>(X, ld, *seqs, B, T, nh, nkv, hd, theta, per);
+    return check_launch("lt_rope_append_rows");
 }
 
 extern "C" int lt_append_kv_rows(float* kbase, const float* ksrc, float* vbase, const float* vsrc, int src_ld, int* len,
@@ -872,4 +956,33 @@ extern "C" int lt_attn_prefill(const float* Q, int q_ld, const float* K, const f
     cudaStream_t s = (cudaStream_t)stream;
     if (hd == 64) return pick_attn_prefill<64>(Q, q_ld, K, V, len, OUT, out_ld, nh, nkv, scale, nrows, maxt, s);
     return pick_attn_prefill<128>(Q, q_ld, K, V, len, OUT, out_ld, nh, nkv, scale, nrows, maxt, s);
+}
+
+extern "C" int lt_attn_prefill_rows(const float* Q, int q_ld, const lt_row_seqs* seqs, int B, int T, float* OUT, int out_ld, int hd,
+                                    int nh, int nkv, float scale, void* stream) {
+    int rc = check_seqs("lt_attn_prefill_rows", seqs, B, T);
+    if (rc != LT_OK) return rc;
+    int maxt = 0;
+    AttnSeqs S = {};
+    bool ok = Q && OUT && (hd == 64 || hd == 128) && nh > 0 && nkv > 0 && nh % nkv == 0 && q_ld >= nh * hd && out_ld >= nh * hd &&
+              q_ld % 4 == 0 && out_ld % 2 == 0 && (reinterpret_cast<uintptr_t>(OUT) & 7u) == 0 && aligned16(Q);
+    for (int b = 0; b < B; b++) {
+        S.k[b] = seqs->k[b];
+        S.v[b] = seqs->v[b];
+        S.total[b] = seqs->start[b] + T;
+        if (S.total[b] > maxt) maxt = S.total[b];
+        ok = ok && aligned16(S.k[b]) && (reinterpret_cast<uintptr_t>(S.v[b]) & 7u) == 0;
+    }
+    cudaStream_t s = (cudaStream_t)stream;
+    if (ok && maxt <= 12000) {
+        rc = hd == 64 ? pick_attn_prefill_rows<64>(Q, q_ld, S, B, OUT, out_ld, nh, nkv, scale, T, maxt, s)
+                      : pick_attn_prefill_rows<128>(Q, q_ld, S, B, OUT, out_ld, nh, nkv, scale, T, maxt, s);
+        if (rc != LT_ERR_UNSUPPORTED) return rc;
+    }
+    for (int b = 0; b < B; b++) {      // short chunks, and what is refused: one at a time
+        rc = lt_attn_prefill(Q + (long)b * T * q_ld, q_ld, S.k[b], S.v[b], seqs->len[b], OUT + (long)b * T * out_ld, out_ld, hd, nh, nkv,
+                             scale, T, S.total[b], stream);
+        if (rc != LT_OK) return rc;
+    }
+    return LT_OK;
 }

@@ -1,6 +1,8 @@
 """The llama / qwen2 block with Q8_0 weights: attention with rotary positions over an fp32 KV cache, gated
 feed-forward.  One token: bpd/lib/dev_residency.py:1381-1477 per layer, every op a launch of the per-op interface
 (`dev_residency`); a prompt portion: the same arithmetic on all rows at once, GEMMs on the tensor cores."""
+import ctypes
+
 import numpy as np
 import torch
 
@@ -120,17 +122,21 @@ class Q8Block(archs.Architecture):
         _lib.call("lt_quant_q8", h.data_ptr(), xq.data_ptr(), xd.data_ptr(), E, R, s())
         Wqkv, bcat, _ = dr._fused_qkv_weight(w, p)
         gemm(Wqkv, E, nq + 2 * nk, qkv, None if bcat is None else dr._dev_const(bcat), 0)
-        for b, c in enumerate(caches):
-            lp = c._ensure_len_ptr(seed=True)
+        for c in caches:
+            if dr._capturing():
+                raise RuntimeError("length seeding during graph capture")
+            c._ensure_len_ptr(seed=False)
             if c.length + T > c.max_seq:
                 raise RuntimeError(f"KV cache overflow: {c.length}+{T} > {c.max_seq}")
-            rows = qkv[b * T:(b + 1) * T]
-            _lib.call("lt_rope_rows", rows.data_ptr(), nq + 2 * nk, lp, T, nh + nkv, hd, theta, s())
-            _lib.call("lt_append_kv_rows", c.k_ptr, rows.data_ptr() + nq * 4, c.v_ptr,
-                      rows.data_ptr() + (nq + nk) * 4, nq + 2 * nk, lp, c.width, c.max_seq, T, 1, s())
-            c.length += T
-            _lib.call("lt_attn_prefill", rows.data_ptr(), nq + 2 * nk, c.k_ptr, c.v_ptr, lp,
-                      att[b * T:(b + 1) * T].data_ptr(), nq, hd, nh, nkv, scale, T, c.length, s())
+        for b in range(0, B, _lib.ROW_SEQS):
+            some = caches[b:b + _lib.ROW_SEQS]
+            seqs = _lib.RowSeqs()
+            for i, c in enumerate(some):
+                seqs.k[i], seqs.v[i], seqs.len[i], seqs.start[i], seqs.max_seq[i] = c.k_ptr, c.v_ptr, c.len_ptr, c.length, c.max_seq
+                c.length += T
+            rows, to = qkv.data_ptr() + 4 * b * T * (nq + 2 * nk), att.data_ptr() + 4 * b * T * nq
+            _lib.call("lt_rope_append_rows", rows, nq + 2 * nk, ctypes.byref(seqs), len(some), T, nh, nkv, hd, theta, s())
+            _lib.call("lt_attn_prefill_rows", rows, nq + 2 * nk, ctypes.byref(seqs), len(some), T, to, nq, hd, nh, nkv, scale, s())
         _lib.call("lt_quant_q8", att.data_ptr(), xq.data_ptr(), xd.data_ptr(), nq, R, s())
         gemm(dr._np(w[f"{p}.attn_output.weight"]), nq, E, x1, x.data_ptr(), E)
         _lib.call("lt_rmsnorm", x1.data_ptr(), dr._dev_const(dr._np(w[f"{p}.ffn_norm.weight"])), h.data_ptr(),
