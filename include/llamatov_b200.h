@@ -465,6 +465,8 @@ int lt_token_record(const int* tok, int* history, int* step, int capacity, void*
  * h_tok to d_tok, launches graph_exec (a cudaGraphExec_t whose step reads d_tok and leaves the chosen token in
  * d_out), copies d_out to page-locked h_out and waits for the stream.  One call per token. */
 int lt_graph_replay_token(void* graph_exec, void* stream, const int* h_tok, int* d_tok, const int* d_out, int* h_out);
+/* The same for a caller that wants the step's n logits: d_logits to h_logits, page-locked or not. */
+int lt_graph_replay_logits(void* graph_exec, void* stream, const int* h_tok, int* d_tok, const float* d_logits, float* h_logits, long n);
 
 #ifdef __cplusplus
 }

@@ -50,6 +50,7 @@ SIGNATURES = {
     "lt_embed_q8": [_vp, _vp, _vp, _vp, _i, _i, _vp],
     "lt_token_record": [_vp, _vp, _vp, _i, _vp],
     "lt_graph_replay_token": [_vp, _vp, _vp, _vp, _vp, _vp],
+    "lt_graph_replay_logits": [_vp, _vp, _vp, _vp, _vp, _vp, ctypes.c_long],
     "lt_embed_q8_rows": [_vp, _vp, _vp, _vp, _i, _i, _i, _vp],
     "lt_rope_rows": [_vp, _i, _vp, _i, _i, _i, _f, _vp],
     "lt_append_kv_rows": [_vp, _vp, _vp, _vp, _i, _vp, _i, _i, _i, _i, _vp],
@@ -158,7 +159,7 @@ _DENSE_QUERIES = {"lt_dn_gqa_step_ws": ([_i, _i, _i], ctypes.c_long),
                   "lt_dn_recurrence_chunked_ws": ([_i, _i, _i, _i], ctypes.c_long)}
 # what the common library exports (the Q8_0 library passes these through to its users as well)
 _COMMON_NAMES = ("lt_last_error", "lt_version", "lt_launch_count", "lt_set_chained_launch", "lt_device_status",
-                 "lt_graph_replay_token", "lt_token_record", "lt_quant_q8", "lt_silu_mul_quant", "lt_silu_mul", "lt_add",
+                 "lt_graph_replay_token", "lt_graph_replay_logits", "lt_token_record", "lt_quant_q8", "lt_silu_mul_quant", "lt_silu_mul", "lt_add",
                  "lt_rmsnorm", "lt_rmsnorm_quant", "lt_rope", "lt_append_kv", "lt_incr_len", "lt_argmax_scratch_bytes",
                  "lt_argmax", "lt_embed_q8")
 

@@ -296,6 +296,17 @@ extern "C" int lt_graph_replay_token(void* graph_exec, void* stream, const int* 
     return LT_OK;
 }
 
+extern "C" int lt_graph_replay_logits(void* graph_exec, void* stream, const int* h_tok, int* d_tok, const float* d_logits, float* h_logits,
+                                      long n) {
+    LT_REQUIRE(graph_exec && h_tok && d_tok && d_logits && h_logits && n > 0, "lt_graph_replay_logits: bad argument");
+    cudaStream_t s = (cudaStream_t)stream;
+    LT_CUDA(cudaMemcpyAsync(d_tok, h_tok, sizeof(int), cudaMemcpyHostToDevice, s));
+    LT_CUDA(cudaGraphLaunch((cudaGraphExec_t)graph_exec, s));
+    LT_CUDA(cudaMemcpyAsync(h_logits, d_logits, (size_t)n * sizeof(float), cudaMemcpyDeviceToHost, s));
+    LT_CUDA(cudaStreamSynchronize(s));
+    return LT_OK;
+}
+
 extern "C" int lt_token_record(const int* tok, int* history, int* step, int capacity, void* stream) {
     LT_REQUIRE(tok && history && step && capacity > 0, "lt_token_record: bad argument");
     k_token_record<<<1, 32, 0, (cudaStream_t)stream>>>(tok, history, step, capacity);

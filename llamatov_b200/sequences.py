@@ -69,6 +69,8 @@ class Sequences:
         s.length += n
         if not len(want):
             return None
+        if n == 1 and len(want) == 1:
+            return out[0].reshape(1, -1)
         return torch.stack([out[int(p)] for p in want])
 
     def _one(self, s, tok):
