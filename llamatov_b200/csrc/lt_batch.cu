@@ -13,6 +13,8 @@
 // The KV caches of the batch are one buffer per layer, [B][max_seq][nkv*hd], with a device
 // length per sequence.
 #include "lt_common.cuh"
+#include <type_traits>
+
 #include "lt_device_ops.cuh"
 
 namespace lt {
@@ -311,6 +313,100 @@ k_attn_pv(const float* __restrict__ P, int s_ld, const float* __restrict__ V, co
         const long col = (long)h * hd + d0 + dl;
         Xq[(long)b * nh * hd + col] = (int8_t)q;
         if (dl == 0) Xd[((long)b * nh * hd + col) >> 5] = dh;
+    }
+}
+
+// The same where (sequence, KV head) pairs are many: a warp takes 64 output elements of all REP heads, a lane two elements of each,
+// so that a value of V is read once for all heads and the chains of a lane overlap (12 shared-memory cycles a position and KV head
+// of 128 instead of 32).  32 sequences of 1024 positions, 32 heads on 8 of 128: 37 us, 27 here (134 MB of values: 21 us).
+constexpr int PW_ROWS = 32, PW_STAGES = 4;
+template <int REP>
+__global__ void __launch_bounds__(32)
+k_attn_pv_warp(const float* __restrict__ P, int s_ld, const float* __restrict__ V, const int* __restrict__ lens,
+               const float* __restrict__ Z, float* __restrict__ OUT, int out_ld, int hd, int nh, int nkv, int max_seq,
+               int8_t* __restrict__ Xq, __half* __restrict__ Xd) {
+    chain_release();
+    chain_wait();
+    __shared__ __align__(16) float vt[PW_STAGES][PW_ROWS][64];
+    __shared__ __align__(16) float pt[PW_STAGES][REP][PW_ROWS];
+    const int b = blockIdx.z, hk = blockIdx.y, lane = threadIdx.x, d0 = blockIdx.x * 64;
+    int L = lens[b];
+    L = L < 0 ? 0 : (L > max_seq ? max_seq : L);
+    const float* Vb = V + ((long)b * max_seq * nkv + hk) * hd + d0;
+    const long vs = (long)nkv * hd;
+    const float* Pb = P + ((long)b * nh + (long)hk * REP) * s_ld;
+    const int tiles = (L + PW_ROWS - 1) / PW_ROWS;
+    auto stage = [&](int k) {   // always commits a group, so that group k is tile k
+        if (k < tiles) {
+            const int buf = k % PW_STAGES, t0 = k * PW_ROWS;
+#pragma unroll
+            for (int i = lane; i < PW_ROWS * 16; i += 32) {
+                const int row = i >> 4, c = i & 15;
+                if (t0 + row < L) cp_async16(&vt[buf][row][c * 4], Vb + (long)(t0 + row) * vs + c * 4);
+            }
+#pragma unroll
+            for (int i = lane; i < REP * (PW_ROWS / 4); i += 32) {
+                const int r = i / (PW_ROWS / 4), c = i - r * (PW_ROWS / 4);
+                if (t0 + c * 4 < L) cp_async16(&pt[buf][r][c * 4], Pb + (long)r * s_ld + t0 + c * 4);
+            }
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    float a[REP], e[REP];
+#pragma unroll
+    for (int r = 0; r < REP; r++) a[r] = e[r] = 0.0f;
+    for (int k = 0; k < PW_STAGES - 1; k++) stage(k);
+    for (int k = 0; k < tiles; k++) {
+        asm volatile("cp.async.wait_group %0;" ::"n"(PW_STAGES - 2) : "memory");
+        __syncwarp();           // tile k is here for all lanes, and all have folded tile k - 1
+        stage(k + PW_STAGES - 1);
+        const int buf = k % PW_STAGES;
+        const int n = L - k * PW_ROWS < PW_ROWS ? L - k * PW_ROWS : PW_ROWS;
+        const float* vc = &vt[buf][0][2 * lane];
+        int t = 0;
+#pragma unroll 2
+        for (; t + 4 <= n; t += 4) {
+            float2 v[4];
+#pragma unroll
+            for (int u = 0; u < 4; u++) v[u] = *(const float2*)(vc + (t + u) * 64);
+            float4 p[REP];
+#pragma unroll
+            for (int r = 0; r < REP; r++) p[r] = *(const float4*)&pt[buf][r][t];
+#pragma unroll
+            for (int r = 0; r < REP; r++) { a[r] = __fmaf_rn(p[r].x, v[0].x, a[r]); e[r] = __fmaf_rn(p[r].x, v[0].y, e[r]); }
+#pragma unroll
+            for (int r = 0; r < REP; r++) { a[r] = __fmaf_rn(p[r].y, v[1].x, a[r]); e[r] = __fmaf_rn(p[r].y, v[1].y, e[r]); }
+#pragma unroll
+            for (int r = 0; r < REP; r++) { a[r] = __fmaf_rn(p[r].z, v[2].x, a[r]); e[r] = __fmaf_rn(p[r].z, v[2].y, e[r]); }
+#pragma unroll
+            for (int r = 0; r < REP; r++) { a[r] = __fmaf_rn(p[r].w, v[3].x, a[r]); e[r] = __fmaf_rn(p[r].w, v[3].y, e[r]); }
+        }
+        for (; t < n; t++) {
+            const float2 v = *(const float2*)(vc + t * 64);
+#pragma unroll
+            for (int r = 0; r < REP; r++) { a[r] = __fmaf_rn(pt[buf][r][t], v.x, a[r]); e[r] = __fmaf_rn(pt[buf][r][t], v.y, e[r]); }
+        }
+    }
+    asm volatile("cp.async.wait_all;" ::: "memory");
+    __syncwarp();
+    float* o = &vt[0][0][0];    // [REP][64], to store and quantise blocks of 32 neighbours
+#pragma unroll
+    for (int r = 0; r < REP; r++) {
+        const float z = Z[(long)b * nh + hk * REP + r];
+        o[r * 64 + 2 * lane] = __fdiv_rn(a[r], z);
+        o[r * 64 + 2 * lane + 1] = __fdiv_rn(e[r], z);
+    }
+    __syncwarp();
+    for (int g = 0; g < 2 * REP; g++) {
+        const float v = o[g * 32 + lane];
+        const long col = (long)(hk * REP + (g >> 1)) * hd + d0 + (g & 1) * 32 + lane;
+        OUT[(long)b * out_ld + col] = v;
+        if (Xq != nullptr) {
+            __half dh;
+            const int q = quant_lane(v, &dh);
+            Xq[(long)b * nh * hd + col] = (int8_t)q;
+            if (lane == 0) Xd[((long)b * nh * hd + col) >> 5] = dh;
+        }
     }
 }
 
@@ -624,6 +720,21 @@ extern "C" long lt_attn_decode_batch_scratch_floats(int nh, int max_seq, int B) 
     return (long)B * nh * s_ld + (long)B * nh;
 }
 
+// f with the number of query heads per KV head as a constant
+template <class F>
+static cudaError_t with_rep(int rep, F f) {
+    switch (rep) {
+        case 1: return f(std::integral_constant<int, 1>());
+        case 2: return f(std::integral_constant<int, 2>());
+        case 3: return f(std::integral_constant<int, 3>());
+        case 4: return f(std::integral_constant<int, 4>());
+        case 5: return f(std::integral_constant<int, 5>());
+        case 6: return f(std::integral_constant<int, 6>());
+        case 7: return f(std::integral_constant<int, 7>());
+        default: return f(std::integral_constant<int, 8>());
+    }
+}
+
 extern "C" int lt_attn_decode_batch(const float* Q, int q_ld, const float* K, const float* V, const int* lens,
                                     float* OUT, int out_ld, float* scratch, int hd, int nh, int nkv, float scale,
                                     int max_seq, int B, int8_t* Xq, uint16_t* Xd, void* stream) {
@@ -657,7 +768,17 @@ extern "C" int lt_attn_decode_batch(const float* Q, int q_ld, const float* K, co
         e = launch_chained(k_attn_softmax, dim3(nh, B), dim3(BT), (size_t)max_seq * sizeof(float), s, S, s_ld, lens, Z, nh,
                            max_seq);
     if (e == cudaSuccess) {
-        if ((long)(hd / 32) * nkv * B >= 592)
+        // A warp per 64 elements needs CTAs enough, and rows long enough for its ring; with one query head per KV head it has the
+        // other form's CTAs and longer reads.  32 heads on 8 of 128, 1024 positions, 8 sequences (128 CTAs) 41 us against 30, 12
+        // (192) 46.8, 47.7, 24 59, 64, 32 67, 76; 500 positions 12 sequences 28.2, 27.8, 24 35, 37; 100 positions 32 sequences
+        // 15.8, 15.3.  8 heads on 8 of 128, 1024 positions: 24 us against 28 for one sequence, 37 against 62 for 16.
+        const long ctas = (long)(hd / 64) * nkv * B;
+        if (hd % 64 == 0 && (rep == 1 || (ctas >= 192 && ctas * max_seq >= 150000)))
+            e = with_rep(rep, [&](auto r) {
+                return launch_chained(k_attn_pv_warp<decltype(r)::value>, dim3(hd / 64, nkv, B), dim3(32), 0, s, S, s_ld, V, lens, Z, OUT, out_ld, hd,
+                                      nh, nkv, max_seq, Xq, (__half*)Xd);
+            });
+        else if ((long)(hd / 32) * nkv * B >= 592)
             e = launch_chained(k_attn_pv<2, 64>, dim3(hd / 32, nkv, B), dim3(32 * rep), pv_smem(2, 64), s, S, s_ld, V, lens, Z, OUT,
                                out_ld, hd, nh, nkv, max_seq, Xq, (__half*)Xd);
         else
