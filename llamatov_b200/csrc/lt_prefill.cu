@@ -557,12 +557,11 @@ static int launch_attn_prefill_wide(const float* Q, int q_ld, const AttnSeqs& S,
 // 16-row form above spends its time on is operand reads (6 of 16 bytes per 32 multiply-adds, 256 of 512 threads
 // folding, one CTA per SM, phases between barriers).  Here a thread owns 4 rows x 4 positions, then 4 rows x HD / 16
 // elements: 8 reads, 4 of them nearly broadcasts, per 64 multiply-adds, and CTAs overlap on an SM (four with heads of 64,
-// two with heads of 128: 52 and 93 KB of shared memory).  Scores are computed twice, first for the row maxima alone: no SM
-// holds 32 rows of scores beside the tiles, and nothing depends on Lmax.  A row's 64 softmax lanes are the 64 positions of
-// a tile, so the lane sums of the denominator stay in the registers of the threads that make the probabilities.  Bound by the operand reads and issue slots of its three
-// products of Lmax^2 / 2 x HD per head (2048 positions: shared memory 74 % busy, issue slots 70 %, FMA pipe 49 %) and by the
-// uneven lengths of the rows.
-// 2048 positions: 14 heads on 2 of 64: 505 us with 16 rows, now 347; 32 heads on 8 of 128: 3273, now 1549.
+// two with heads of 128: 52 and 93 KB of shared memory).  The row maxima come first, by bounds from the tensor
+// cores: no SM holds 32 rows of scores beside the tiles, and nothing depends on Lmax.  A row's 64 softmax lanes are the 64 positions of
+// a tile, so the lane sums of the denominator stay in the registers of the threads that make the probabilities.  Bound by the operand reads (twice the clocks of the
+// multiply-adds) and issue slots of its two exact products of Lmax^2 / 2 x HD per head and by the uneven lengths of the rows.
+// 2048 positions: 14 heads on 2 of 64: 505 us with 16 rows, now 306; 32 heads on 8 of 128: 3273, now 1275.
 // (64 rows per CTA, 8 x 4 per thread: 444; the 448 CTAs are all resident at once and share the SMs unevenly.)
 constexpr int PB_TILE = 64;
 
@@ -575,7 +574,7 @@ struct PrefillBlock {
 };
 
 template <int HD, int QT>
-__global__ void __launch_bounds__(PrefillBlock<HD, QT>::THREADS)
+__global__ void __launch_bounds__(PrefillBlock<HD, QT>::THREADS, HD == 64 ? 4 : 2)
 k_attn_prefill_block(const float* __restrict__ Q, int q_ld, const __grid_constant__ AttnSeqs S, int nseq, float* __restrict__ OUT, int out_ld,
                      int nh, int nkv, float scale, int nrows, int maxt, int* status) {
     using B = PrefillBlock<HD, QT>;
@@ -660,11 +659,165 @@ k_attn_prefill_block(const float* __restrict__ Q, int q_ld, const __grid_constan
 #pragma unroll
     for (int i = 0; i < MQ; i++) lim[i] = L0 + r0 + m * MQ + i + 1;
 
-    // ---- row maxima
+    // ---- row maxima.  Only the greatest score of a row is wanted here, and it need be exact only there: bf16 products on the
+    // tensor cores (mma: a sixteenth of the shared-memory reads of the blocked product) are within eps = |q| |k| |scale| 2^-8 x 1.5
+    // of every score (both operands rounded to 8 bits, 2^-9 each; 2^-10 for the place below; the rest for the rounding of the sums,
+    // below 2^-15, and of eps itself), so product + eps bounds a score from above.  A thread sees a sixteenth of a row's positions
+    // and keeps the three greatest bounds, the place in the low 13 bits of each.  The declared chain of every warp's greatest gives
+    // a score that the maximum reaches at least; what else may reach it (one or two of a row, from the first two of a thread) is
+    // folded too.  Where a third may, or many do (rows of equal scores), or eps is no bound (a norm or the scale not finite, or near
+    // overflow), the blocked product finds the maxima, 12 % more time in all than without this search.
+    // 2048 positions, us: 14 heads of 64 338 -> 306, 32 heads of 128 1604 -> 1275.  (Products in tf32: 406; candidates found by a
+    // second walk over K: 350.)
     float mx[MQ];
 #pragma unroll
     for (int i = 0; i < MQ; i++) mx[i] = -1e30f;
-    for (int t0 = 0, buf = 0; t0 < Lmax; t0 += PB_TILE, buf ^= 1) {
+    bool blocked = true;
+    if (Lmax <= PB_TILE * 2048) {
+        static_assert(QT == 32 && PB_THREADS == 128 && PB_TILE == 64, "a warp takes 16 positions of a tile for 32 rows");
+        constexpr int NCAND = 2 * PB_THREADS;    // one for each warp and row, as many others
+        const int w = tid >> 5, g = (tid & 31) >> 2, t4 = tid & 3;
+        int* mk = (int*)ps;                      // [QT] greatest exact score, as an ordered integer
+        int* ncand = mk + QT;
+        int* list = ncand + 4;                   // [NCAND] candidates: position * 32 + row
+        static_assert(QT + 4 + NCAND <= QT * PST, "candidates beside the maxima");
+        auto ordered = [](int v) { return v ^ ((v >> 31) & 0x7fffffff); };
+        auto bf16 = [](float lo, float hi) {
+            unsigned r;
+            asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(r) : "f"(hi), "f"(lo));
+            return r;
+        };
+        auto chain = [&](int at) {
+            const int r = at & 31;
+            const float4* q4 = (const float4*)(qs + r * ST);
+            const float4* k4 = (const float4*)(K + (long)hk * HD + (long)(at >> 5) * rstride);
+            float v = 0.0f;
+#pragma unroll 8
+            for (int d = 0; d < HD / 4; d++) {
+                const float4 q = q4[d], k = __ldg(k4 + d);
+                v = __fmaf_rn(q.x, k.x, v); v = __fmaf_rn(q.y, k.y, v);
+                v = __fmaf_rn(q.z, k.z, v); v = __fmaf_rn(q.w, k.w, v);
+            }
+            atomicMax(mk + r, ordered(__float_as_int(__fmul_rn(v, scale))));
+        };
+        list[tid] = -1;
+        if (tid < QT) mk[tid] = ordered(__float_as_int(-1e30f));
+        if (tid == 0) *ncand = 0;
+        __syncthreads();                         // the q rows are stored
+        // Fragments: thread t4 of a row's four holds elements 16 c + 4 t4 .. + 3 (a sum may take the elements in any order as
+        // long as both operands agree).
+        unsigned qa[HD / 16][2][2][2];           // [16 elements][16 rows][row g or g + 8][pair]
+        float qn[4] = {0.0f, 0.0f, 0.0f, 0.0f};  // squared norms of rows g + 8 i, then eps / |k|
+#pragma unroll
+        for (int c = 0; c < HD / 16; c++)
+#pragma unroll
+            for (int i = 0; i < 4; i++) {
+                const float4 q = *(const float4*)(qs + (g + 8 * i) * ST + 16 * c + 4 * t4);
+                qn[i] += q.x * q.x + q.y * q.y + q.z * q.z + q.w * q.w;
+                qa[c][i >> 1][i & 1][0] = bf16(q.x, q.y);
+                qa[c][i >> 1][i & 1][1] = bf16(q.z, q.w);
+            }
+        float top[4][3];                         // rows g + 8 i
+        bool bad = false;
+#pragma unroll
+        for (int i = 0; i < 4; i++) {
+            qn[i] += __shfl_xor_sync(0xffffffffu, qn[i], 1);
+            qn[i] += __shfl_xor_sync(0xffffffffu, qn[i], 2);
+            bad = bad || !(qn[i] < 1e37f);
+            qn[i] = sqrtf(fmaxf(qn[i], 1e-30f)) * fabsf(scale) * (1.5f / 256.0f);
+            bad = bad || !(qn[i] < 1e14f);
+            top[i][0] = top[i][1] = top[i][2] = -1e38f;
+        }
+        for (int t0 = 0, buf = 0; t0 < Lmax; t0 += PB_TILE, buf ^= 1) {
+            if (t0 + PB_TILE < Lmax) {
+                copy_tile(K, t0 + PB_TILE, buf ? tk : tv);
+                asm volatile("cp.async.wait_group 1;" ::: "memory");
+            } else {
+                asm volatile("cp.async.wait_group 0;" ::: "memory");
+            }
+            __syncthreads();
+            const float* kt = (buf ? tv : tk) + (w * 16 + g) * ST + 4 * t4;
+            const bool edge = t0 + PB_TILE > L0 + r0 + 1 || nq < QT;
+            const int tp = t0 + w * 16 + 2 * t4 - (L0 + r0 + g);
+#pragma unroll
+            for (int y = 0; y < 2; y++) {        // eight positions
+                float c[2][4], k2 = 0.0f;
+#pragma unroll
+                for (int x = 0; x < 2; x++)
+#pragma unroll
+                    for (int e = 0; e < 4; e++) c[x][e] = 0.0f;
+#pragma unroll
+                for (int cc = 0; cc < HD / 16; cc++) {
+                    const float4 k = *(const float4*)(kt + y * 8 * ST + 16 * cc);
+                    k2 += k.x * k.x + k.y * k.y + k.z * k.z + k.w * k.w;
+                    const unsigned k0 = bf16(k.x, k.y), k1 = bf16(k.z, k.w);
+#pragma unroll
+                    for (int x = 0; x < 2; x++)
+                        asm("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
+                            : "+f"(c[x][0]), "+f"(c[x][1]), "+f"(c[x][2]), "+f"(c[x][3])
+                            : "r"(qa[cc][x][0][0]), "r"(qa[cc][x][1][0]), "r"(qa[cc][x][0][1]), "r"(qa[cc][x][1][1]), "r"(k0), "r"(k1));
+                }
+                k2 += __shfl_xor_sync(0xffffffffu, k2, 1);
+                k2 += __shfl_xor_sync(0xffffffffu, k2, 2);
+                bad = bad || !(k2 < 1e37f);
+                const float kg = sqrtf(fmaxf(k2, 1e-30f));       // of position g; the products are those of positions 2 t4 and 2 t4 + 1
+                const float kn[2] = {__shfl_sync(0xffffffffu, kg, 8 * t4), __shfl_sync(0xffffffffu, kg, 8 * t4 + 4)};
+#pragma unroll
+                for (int x = 0; x < 2; x++)
+#pragma unroll
+                    for (int e = 0; e < 4; e++) {
+                        const int i = 2 * x + (e >> 1);
+                        float v = __fmaf_rn(c[x][e], scale, __fmaf_rn(qn[i], kn[e & 1], 1e-37f));
+                        if (edge && !(tp + 8 * y + (e & 1) <= 8 * i && g + 8 * i < nq)) v = -1e38f;
+                        v = __int_as_float((__float_as_int(v) & ~0x1fff) | (t0 / PB_TILE * 4 + 2 * y + (e & 1)));
+                        float(&a)[3] = top[i];
+                        const float d0 = fminf(a[0], v);
+                        a[0] = fmaxf(a[0], v);
+                        const float d1 = fminf(a[1], d0);
+                        a[1] = fmaxf(a[1], d0);
+                        a[2] = fmaxf(a[2], d1);
+                    }
+            }
+            __syncthreads();                     // the tile may be replaced
+        }
+        auto position = [&](float v) {
+            const int place = __float_as_int(v) & 0x1fff;
+            return (place >> 2) * PB_TILE + w * 16 + (place & 2) * 4 + 2 * t4 + (place & 1);
+        };
+        // the greatest bound of the warp, where it sees a position of the row at all (of several threads with it, one)
+#pragma unroll
+        for (int i = 0; i < 4; i++) {
+            float v = fmaxf(top[i][0], __shfl_xor_sync(0xffffffffu, top[i][0], 1));
+            v = fmaxf(v, __shfl_xor_sync(0xffffffffu, v, 2));
+            if (top[i][0] == v && v > -9e37f) list[w * QT + g + 8 * i] = position(v) * 32 + g + 8 * i;
+        }
+        blocked = __syncthreads_or(bad);
+        if (!blocked) {
+            if (list[tid] >= 0) chain(list[tid]);
+            __syncthreads();
+#pragma unroll
+            for (int i = 0; i < 4; i++) {
+                const float least = __int_as_float(ordered(mk[g + 8 * i]));
+                bad = bad || top[i][2] >= least;
+#pragma unroll
+                for (int j = 0; j < 2; j++)
+                    if (top[i][j] >= least && !(j == 0 && list[w * QT + g + 8 * i] == position(top[i][0]) * 32 + g + 8 * i)) {
+                        const int at = atomicAdd(ncand, 1);
+                        if (at < NCAND - PB_THREADS) list[PB_THREADS + at] = position(top[i][j]) * 32 + g + 8 * i;
+                    }
+            }
+            blocked = __syncthreads_or(bad) || *ncand > NCAND - PB_THREADS;
+        }
+        if (!blocked) {
+            if (tid < *ncand) chain(list[PB_THREADS + tid]);
+            __syncthreads();
+#pragma unroll
+            for (int i = 0; i < MQ; i++) mx[i] = fmaxf(mx[i], __int_as_float(ordered(mk[m * MQ + i])));
+        } else {
+            copy_tile(K, 0, tk);
+        }
+    }
+    for (int t0 = 0, buf = 0; blocked && t0 < Lmax; t0 += PB_TILE, buf ^= 1) {
         if (t0 + PB_TILE < Lmax) {
             copy_tile(K, t0 + PB_TILE, buf ? tk : tv);
             asm volatile("cp.async.wait_group 1;" ::: "memory");
@@ -828,11 +981,11 @@ static int pick_attn_prefill_rows(const float* Q, int q_ld, const AttnSeqs& S, i
     bool aligned = true;
     for (int b = 0; b < nseq; b++) aligned = aligned && aligned16(S.v[b]);
     if (nrows >= 32 && aligned) {
-        // 32 rows per CTA from three CTAs for each SM on; below, smaller tiles fill the SMs better.  Heads of 64, 14 of them:
-        // 333 rows (154 CTAs) 28 us with 16 rows per CTA, 37 with 32, 850 rows (378) 112 either way, 1200 rows (532) 196 and 183.
-        // Heads of 128 cross between 320 and 450 CTAs: 16 heads, 600 rows (304) 118 and 122, 700 rows (352) 151 and 139;
-        // 32 heads behind 700 positions, 400 rows (416) 359 and 376, 448 rows (448) 404 and 389 ...
-        if ((long)((nrows + 31) / 32) * nh * nseq >= 3L * sm_count())
+        // 32 rows per CTA from two CTAs (heads of 64) or 9/4 (heads of 128) for each SM on; below, smaller tiles fill the SMs
+        // better.  us with 16 and with 32 rows per CTA: 14 heads of 64, 333 rows (154 CTAs) 31 and 36, 500 (224) 52 and 60, 600 (266)
+        // 67 and 62, 700 (308) 84 and 79, 850 (378) 115 and 97; of 128, 16 heads, 600 rows (304) 121 and 125, 32 heads, 300 rows
+        // (320) 74 and 67, 400 behind 700 positions (416) 358 and 346.
+        if ((long)((nrows + 31) / 32) * nh * nseq * 4 >= (HD == 64 ? 8L : 9L) * sm_count())
             return launch_attn_prefill_block<HD, 32>(Q, q_ld, S, nseq, OUT, out_ld, nh, nkv, scale, nrows, maxt, s);
         // ... where the score rows of 16 queries fit one SM beside double-buffered tiles
         if (attn_prefill_wide_smem<HD>(maxt) <= 227 * 1024)
