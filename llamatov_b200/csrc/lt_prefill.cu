@@ -561,7 +561,7 @@ static int launch_attn_prefill_wide(const float* Q, int q_ld, const AttnSeqs& S,
 // cores: no SM holds 32 rows of scores beside the tiles, and nothing depends on Lmax.  A row's 64 softmax lanes are the 64 positions of
 // a tile, so the lane sums of the denominator stay in the registers of the threads that make the probabilities.  Bound by the operand reads (twice the clocks of the
 // multiply-adds) and issue slots of its two exact products of Lmax^2 / 2 x HD per head and by the uneven lengths of the rows.
-// 2048 positions: 14 heads on 2 of 64: 505 us with 16 rows, now 306; 32 heads on 8 of 128: 3273, now 1275.
+// 2048 positions: 14 heads on 2 of 64: 505 us with 16 rows, now 305; 32 heads on 8 of 128: 3273, now 1269.
 // (64 rows per CTA, 8 x 4 per thread: 444; the 448 CTAs are all resident at once and share the SMs unevenly.)
 constexpr int PB_TILE = 64;
 
@@ -659,16 +659,21 @@ k_attn_prefill_block(const float* __restrict__ Q, int q_ld, const __grid_constan
 #pragma unroll
     for (int i = 0; i < MQ; i++) lim[i] = L0 + r0 + m * MQ + i + 1;
 
-    // ---- row maxima.  Only the greatest score of a row is wanted here, and it need be exact only there: bf16 products on the
-    // tensor cores (mma: a sixteenth of the shared-memory reads of the blocked product) are within eps = |q| |k| |scale| 2^-8 x 1.5
-    // of every score (both operands rounded to 8 bits, 2^-9 each; 2^-10 for the place below; the rest for the rounding of the sums,
-    // below 2^-15, and of eps itself), so product + eps bounds a score from above.  A thread sees a sixteenth of a row's positions
-    // and keeps the three greatest bounds, the place in the low 13 bits of each.  The declared chain of every warp's greatest gives
-    // a score that the maximum reaches at least; what else may reach it (one or two of a row, from the first two of a thread) is
-    // folded too.  Where a third may, or many do (rows of equal scores), or eps is no bound (a norm or the scale not finite, or near
-    // overflow), the blocked product finds the maxima, 12 % more time in all than without this search.
-    // 2048 positions, us: 14 heads of 64 338 -> 306, 32 heads of 128 1604 -> 1275.  (Products in tf32: 406; candidates found by a
-    // second walk over K: 350.)
+    // ---- row maxima.  Only the greatest score of a row is wanted here, and it need be exact only there: fp16 products on the
+    // tensor cores (mma: a sixteenth of the shared-memory reads of the blocked product) are within eps of every score, so product +
+    // eps bounds a score from above.  With u = 2^-11, the largest relative error of a rounding to 11 bits, and 2^-25, the largest
+    // error of one to a subnormal fp16, the product of the rounded rows is off by at most
+    //     2^-10 (1 + 2^-12) |q| |k| + 2^-25 sqrt(HD) (|q| + |k|) (1 + u) + 2^-50 HD;
+    // its sums and the declared chain's add less than 2^-14 |q| |k|, and the place below, which takes 13 bits of the bound, 2^-10 of
+    // it.  eps = 2.25 x 2^-10 (|q| + 2^-12) (|k| + 2^-12) |scale| is more than all of them (2.07 x 2^-10 |q| |k|; 2^-25 sqrt(128) = 0.63
+    // x 2.25 x 2^-22).  The norms' own rounding is below 2^-16 of eps, and 1e-37 covers products that underflow.
+    // A thread sees a sixteenth of a row's positions and keeps the three greatest bounds, the place in the low 13 bits of each.  The
+    // declared chain of every warp's greatest gives a score that the maximum reaches at least; what else may reach it (one or two of
+    // a row, from the first two of a thread) is folded too.  Where a third may, or many do (rows of equal scores), or eps is no bound
+    // (norms at the end of fp16 or beyond, or not finite), the blocked product finds the maxima.
+    // 2048 positions, us, with the blocked product alone and so: 14 heads of 64 349 and 305, 32 heads of 128 1549 and 1269; keys with
+    // a bias of three times their deviation 349 and 306, of twenty times 349 and 389, equal keys 350 and 418.  (bf16 needs a bound
+    // four times as wide; products in tf32: 406; candidates found by a second walk over K: 350.)
     float mx[MQ];
 #pragma unroll
     for (int i = 0; i < MQ; i++) mx[i] = -1e30f;
@@ -682,9 +687,9 @@ k_attn_prefill_block(const float* __restrict__ Q, int q_ld, const __grid_constan
         int* list = ncand + 4;                   // [NCAND] candidates: position * 32 + row
         static_assert(QT + 4 + NCAND <= QT * PST, "candidates beside the maxima");
         auto ordered = [](int v) { return v ^ ((v >> 31) & 0x7fffffff); };
-        auto bf16 = [](float lo, float hi) {
+        auto fp16 = [](float lo, float hi) {
             unsigned r;
-            asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(r) : "f"(hi), "f"(lo));
+            asm("cvt.rn.f16x2.f32 %0, %1, %2;" : "=r"(r) : "f"(hi), "f"(lo));
             return r;
         };
         auto chain = [&](int at) {
@@ -714,8 +719,8 @@ k_attn_prefill_block(const float* __restrict__ Q, int q_ld, const __grid_constan
             for (int i = 0; i < 4; i++) {
                 const float4 q = *(const float4*)(qs + (g + 8 * i) * ST + 16 * c + 4 * t4);
                 qn[i] += q.x * q.x + q.y * q.y + q.z * q.z + q.w * q.w;
-                qa[c][i >> 1][i & 1][0] = bf16(q.x, q.y);
-                qa[c][i >> 1][i & 1][1] = bf16(q.z, q.w);
+                qa[c][i >> 1][i & 1][0] = fp16(q.x, q.y);
+                qa[c][i >> 1][i & 1][1] = fp16(q.z, q.w);
             }
         float top[4][3];                         // rows g + 8 i
         bool bad = false;
@@ -723,8 +728,8 @@ k_attn_prefill_block(const float* __restrict__ Q, int q_ld, const __grid_constan
         for (int i = 0; i < 4; i++) {
             qn[i] += __shfl_xor_sync(0xffffffffu, qn[i], 1);
             qn[i] += __shfl_xor_sync(0xffffffffu, qn[i], 2);
-            bad = bad || !(qn[i] < 1e37f);
-            qn[i] = sqrtf(fmaxf(qn[i], 1e-30f)) * fabsf(scale) * (1.5f / 256.0f);
+            bad = bad || !(qn[i] < 4e9f);        // no element beyond 63245
+            qn[i] = (sqrtf(qn[i]) + 0x1p-12f) * fabsf(scale) * (2.25f / 1024.0f);
             bad = bad || !(qn[i] < 1e14f);
             top[i][0] = top[i][1] = top[i][2] = -1e38f;
         }
@@ -750,17 +755,17 @@ k_attn_prefill_block(const float* __restrict__ Q, int q_ld, const __grid_constan
                 for (int cc = 0; cc < HD / 16; cc++) {
                     const float4 k = *(const float4*)(kt + y * 8 * ST + 16 * cc);
                     k2 += k.x * k.x + k.y * k.y + k.z * k.z + k.w * k.w;
-                    const unsigned k0 = bf16(k.x, k.y), k1 = bf16(k.z, k.w);
+                    const unsigned k0 = fp16(k.x, k.y), k1 = fp16(k.z, k.w);
 #pragma unroll
                     for (int x = 0; x < 2; x++)
-                        asm("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
+                        asm("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
                             : "+f"(c[x][0]), "+f"(c[x][1]), "+f"(c[x][2]), "+f"(c[x][3])
                             : "r"(qa[cc][x][0][0]), "r"(qa[cc][x][1][0]), "r"(qa[cc][x][0][1]), "r"(qa[cc][x][1][1]), "r"(k0), "r"(k1));
                 }
                 k2 += __shfl_xor_sync(0xffffffffu, k2, 1);
                 k2 += __shfl_xor_sync(0xffffffffu, k2, 2);
-                bad = bad || !(k2 < 1e37f);
-                const float kg = sqrtf(fmaxf(k2, 1e-30f));       // of position g; the products are those of positions 2 t4 and 2 t4 + 1
+                bad = bad || !(k2 < 4e9f);
+                const float kg = sqrtf(k2) + 0x1p-12f;           // of position g; the products are those of positions 2 t4 and 2 t4 + 1
                 const float kn[2] = {__shfl_sync(0xffffffffu, kg, 8 * t4), __shfl_sync(0xffffffffu, kg, 8 * t4 + 4)};
 #pragma unroll
                 for (int x = 0; x < 2; x++)

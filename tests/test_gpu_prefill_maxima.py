@@ -38,3 +38,49 @@ def test_row_maxima_bit_exact(name, hd, nh, nkv, T, L0, scale):
         want = attend(Q[r:], K, V, n, L0 + r + n, hd, nh, nkv, scale)
         assert torch.equal(got[r:r + n].nan_to_num(nan=123.0), want.nan_to_num(nan=123.0)), (name, r)
     assert _lib.device_status() == set()
+
+
+# One large element that q and all keys share, as projections with a bias produce: it takes the rounding error of 16 bits to one side in
+# every key.  Its value is just below the middle of two neighbours with `bits` significant ones, the keys' spread below it.
+def _shared(bits, spread, noise, big=8.0):
+    def edit(q, k, g):
+        q.mul_(noise)
+        k.mul_(noise)
+        q[..., 0] = big * (1 + 0.98 * 2.0 ** -bits)
+        k[..., 0] = big * (1 + 0.98 * 2.0 ** -bits) * (1 - spread * torch.rand(k.shape[:2], device="cuda", generator=g))
+    return edit
+
+
+def _two_keys(bits):      # the greatest score loses most by rounding, the next one nothing
+    def edit(q, k, g):
+        q.zero_()
+        k.zero_()
+        q[..., 0] = 1 + 0.98 * 2.0 ** -bits
+        k[3, :, 0] = 1 + 0.98 * 2.0 ** -bits
+        k[7, :, 0], k[7, :, 1] = 1 + 0.8 * 2.0 ** -bits, 1
+    return edit
+
+
+SIXTEEN = {f"shared-{b}-{s}-{n}": _shared(b, s, n) for b in (8, 11) for s in (2.0 ** -b, 2.0 ** (2 - b), 0.01) for n in (0, 0.05)}
+SIXTEEN |= {f"biased-{b}": _shared(b, 0.002, 1.0, 100.0) for b in (8, 11)} | {f"two-{b}": _two_keys(b) for b in (8, 11)}
+# about half of the elements below the normal fp16; norms just inside and just beyond what fp16 may hold
+TIMES = {"small": (1e-3, 1e-4), "inside": (6e3, 6e3), "beyond": (1e4, 1e4)}
+SIXTEEN |= {n: lambda q, k, g, t=t: (q.mul_(t[0]), k.mul_(t[1])) for n, t in TIMES.items()}
+
+
+@pytest.mark.parametrize("name", SIXTEEN)
+@pytest.mark.parametrize("hd,nh,nkv,T,L0", [(64, 14, 2, 1025, 3), (128, 32, 8, 450, 64)])
+def test_row_maxima_where_sixteen_bits_round_to_one_side(name, hd, nh, nkv, T, L0):
+    g = torch.Generator(device="cuda").manual_seed(T)
+    L = L0 + T
+    Q, K, V = (torch.randn((n, w, hd), device="cuda", generator=g) for n, w in ((T, nh), (L, nkv), (L, nkv)))
+    a, b = TIMES.get(name, (1.0, 1.0))
+    scale = hd ** -0.5 / (a * b)            # scores of ordinary size
+    SIXTEEN[name](Q, K, g)
+    Q, K = Q.reshape(T, -1), K.reshape(L, -1)
+    got = attend(Q, K, V, T, L, hd, nh, nkv, scale)
+    for r in range(0, T, 31):
+        n = min(31, T - r)
+        want = attend(Q[r:], K, V, n, L0 + r + n, hd, nh, nkv, scale)
+        assert torch.equal(got[r:r + n], want), (name, r)
+    assert torch.isfinite(got).all() and _lib.device_status() == set()
