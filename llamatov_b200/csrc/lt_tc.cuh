@@ -4,6 +4,7 @@
 #include <cuda.h>
 
 #include "lt_common.cuh"
+#include "lt_wait.cuh"
 
 namespace lt {
 namespace tc {
@@ -77,17 +78,14 @@ __device__ __forceinline__ bool bar_sleep(unsigned bar, unsigned parity) {
     return ok != 0;
 }
 __device__ __forceinline__ void bar_wait(bool done, unsigned bar, unsigned parity, volatile int* abort_flag, int* status) {
-    if (done || bar_sleep(bar, parity)) return;
-    const long long t0 = clock64();
-    while (!bar_sleep(bar, parity)) {
-        if (*abort_flag) return;
-        if (clock64() - t0 > WAIT_LIMIT) {
-            *abort_flag = 1;
-            atomicOr(status, LT_STATUS_WAIT_TIMEOUT);
-            return;
-        }
-    }
+    if (done) return;
+    bounded_wait([&] { return bar_sleep(bar, parity); }, [] { return (long long)clock64(); }, WAIT_LIMIT, abort_flag, [&] {
+        *abort_flag = 1;
+        atomicOr(status, LT_STATUS_WAIT_TIMEOUT);
+    });
 }
+// for a whole warp: has a wait of the CTA run out of time?
+__device__ __forceinline__ bool gave_up(const volatile int* abort_flag) { return __any_sync(0xffffffffu, *abort_flag != 0); }
 
 // One thread of a converged warp.  Roles whose single thread issues copies or MMAs run their loops as a warp and pick the
 // thread at the instruction: counters and descriptors then stay in uniform registers, which those instructions read.
