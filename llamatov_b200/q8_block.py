@@ -133,9 +133,10 @@ class Q8Block(archs.Architecture):
             seqs = _lib.RowSeqs()
             for i, c in enumerate(some):
                 seqs.k[i], seqs.v[i], seqs.len[i], seqs.start[i], seqs.max_seq[i] = c.k_ptr, c.v_ptr, c.len_ptr, c.length, c.max_seq
-                c.length += T
             rows, to = qkv.data_ptr() + 4 * b * T * (nq + 2 * nk), att.data_ptr() + 4 * b * T * nq
             _lib.call("lt_rope_append_rows", rows, nq + 2 * nk, ctypes.byref(seqs), len(some), T, nh, nkv, hd, theta, s())
+            for c in some:      # not before the rows are accepted: a refused call leaves the lengths as the device has them
+                c.length += T
             _lib.call("lt_attn_prefill_rows", rows, nq + 2 * nk, ctypes.byref(seqs), len(some), T, to, nq, hd, nh, nkv, scale, s())
         _lib.call("lt_quant_q8", att.data_ptr(), xq.data_ptr(), xd.data_ptr(), nq, R, s())
         gemm(dr._np(w[f"{p}.attn_output.weight"]), nq, E, x1, x.data_ptr(), E)
