@@ -292,7 +292,7 @@ int lt_attn_prefill(const float* Q, int q_ld, const float* K, const float* V, co
                     int out_ld, int hd, int nh, int nkv, float scale, int nrows, int maxt, void* stream);
 
 /* Chunks of T new rows of up to LT_ROW_SEQS sequences, one after the other in the rows of a matrix: each has caches of k and v rows
- * (nkv * hd floats, room for max_seq), a device length, and start rows before the chunk. */
+ * (nkv * hd floats, room for max_seq), a device length of its own, and start rows before the chunk. */
 #define LT_ROW_SEQS 8
 typedef struct {
     float* k[LT_ROW_SEQS];

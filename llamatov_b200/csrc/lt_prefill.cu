@@ -1048,6 +1048,7 @@ static int check_seqs(const char* what, const lt_row_seqs* S, int B, int T) {
         LT_REQUIRE(S->k[b] && S->v[b] && S->len[b], "%s: null pointer", what);
         LT_REQUIRE(S->start[b] >= 0 && S->start[b] + (long)T <= S->max_seq[b], "%s: %d + %d positions exceed %d", what, S->start[b], T,
                    S->max_seq[b]);
+        for (int o = 0; o < b; o++) LT_REQUIRE(S->len[o] != S->len[b], "%s: sequences %d and %d have one length", what, o, b);
     }
     return LT_OK;
 }

@@ -128,8 +128,11 @@ class Q8Block(archs.Architecture):
             c._ensure_len_ptr(seed=False)
             if c.length + T > c.max_seq:
                 raise RuntimeError(f"KV cache overflow: {c.length}+{T} > {c.max_seq}")
-        for b in range(0, B, _lib.ROW_SEQS):
-            some = caches[b:b + _lib.ROW_SEQS]
+        b = 0
+        while b < B:
+            some = caches[b:b + 1]          # up to ROW_SEQS a launch; a cache that comes again goes on behind its own rows, in the next
+            while len(some) < _lib.ROW_SEQS and b + len(some) < B and not any(c is caches[b + len(some)] for c in some):
+                some = caches[b:b + len(some) + 1]
             seqs = _lib.RowSeqs()
             for i, c in enumerate(some):
                 seqs.k[i], seqs.v[i], seqs.len[i], seqs.start[i], seqs.max_seq[i] = c.k_ptr, c.v_ptr, c.len_ptr, c.length, c.max_seq
@@ -138,6 +141,7 @@ class Q8Block(archs.Architecture):
             for c in some:      # not before the rows are accepted: a refused call leaves the lengths as the device has them
                 c.length += T
             _lib.call("lt_attn_prefill_rows", rows, nq + 2 * nk, ctypes.byref(seqs), len(some), T, to, nq, hd, nh, nkv, scale, s())
+            b += len(some)
         _lib.call("lt_quant_q8", att.data_ptr(), xq.data_ptr(), xd.data_ptr(), nq, R, s())
         gemm(dr._np(w[f"{p}.attn_output.weight"]), nq, E, x1, x.data_ptr(), E)
         _lib.call("lt_rmsnorm", x1.data_ptr(), dr._dev_const(dr._np(w[f"{p}.ffn_norm.weight"])), h.data_ptr(),

@@ -4,7 +4,7 @@ import ctypes
 import pytest
 import torch
 
-from llamatov_b200 import _lib
+from llamatov_b200 import _lib, dev_residency as dr, prefill, synth
 
 pytestmark = pytest.mark.gpu
 
@@ -51,3 +51,19 @@ def test_rows_that_do_not_fit_are_refused():
     for B in (1, 0, 9):
         with pytest.raises(RuntimeError):
             _lib.call("lt_rope_append_rows", X.data_ptr(), 192, ctypes.byref(seqs), B, 4, 1, 1, 64, 1e4, torch.cuda.current_stream().cuda_stream)
+
+
+def test_one_cache_for_two_portions_of_a_batch():
+    """The second portion continues the first one's context: the bits of one portion of both."""
+    dr.reset_engine_state()
+    dr.apply_production_profile()
+    m = synth.make_model("tiny-qwen64", seed=3)
+    w, cfg = synth.reference_weights(m)
+    toks = torch.randint(0, m["cfg"]["vocab"], (2, 40), generator=torch.Generator().manual_seed(1))
+    one, two = [None] * cfg["n_layers"], [None] * cfg["n_layers"]
+    want = prefill.prefill_resident(w, cfg, toks.reshape(-1), one)
+    got = prefill.prefill_resident(w, cfg, toks, [two, two])
+    assert torch.equal(want.view(torch.int32), got.view(torch.int32))
+    for a, b in zip(one, two):
+        assert a.length == b.length == int(b._len.item()) == 80
+        assert (a.k_slice_host() == b.k_slice_host()).all() and (a.v_slice_host() == b.v_slice_host()).all()

@@ -1,5 +1,6 @@
 """Host side of a prompt portion of the Q8_0 block, the library replaced by a recorder: which rows go to which cache in which launch,
 and what the caches' lengths are afterwards."""
+import ctypes
 from types import SimpleNamespace
 
 import pytest
@@ -63,3 +64,20 @@ def test_ten_sequences_take_two_launches(run):
     a, b = [(1000 * (i + 1), i) for i in range(8)], [(9000, 8), (10000, 9)]
     assert seen == [("rope", a, 0), ("attn", a, 0), ("rope", b, 8 * T), ("attn", b, 8 * T)]
     assert [c.length for c in caches] == [i + T for i in range(10)]
+
+
+def test_a_cache_that_comes_again_goes_on_behind_its_rows(run):
+    a, b = Cache(1, 3), Cache(2, 0)
+    seen = run([a, b, a, a])
+    assert [s for s in seen if s[0] == "rope"] == [("rope", [(1000, 3), (2000, 0)], 0), ("rope", [(1000, 3 + T)], 2 * T), ("rope", [(1000, 3 + 2 * T)], 3 * T)]
+    assert [n for n, *_ in seen] == ["rope", "attn"] * 3 and (a.length, b.length) == (3 + 3 * T, T)
+
+
+def test_the_library_refuses_one_length_for_two_sequences():
+    s = _lib.RowSeqs()
+    for i in range(2):
+        s.k[i] = s.v[i] = s.len[i] = 4096 * (i + 1)
+        s.max_seq[i] = MAX_SEQ
+    s.len[1] = s.len[0]
+    with pytest.raises(RuntimeError, match="one length"):
+        _lib.call("lt_rope_append_rows", 4096, 192, ctypes.byref(s), 2, T, 1, 1, 64, 1e4, None)
