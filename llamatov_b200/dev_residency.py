@@ -1072,6 +1072,7 @@ class GraphRunner:
             c.length = n
         self._assert_weight_cache_frozen()
         self.graph = g
+        self._exec_ptr = None       # the handle of the graph before, which goes with it
         self.captured = True
 
     def _forward_on_device_token(self, tok_dev, out_ptr):
