@@ -231,8 +231,7 @@ k_q8_gemm_res(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ C
             const bool one = elect_one();
             tiles([&](int rt, int tt, int n, bool fresh) {
                 const unsigned buf = n & 1, xf = bars + R_XFULL + 8 * buf;
-                wait(bars + R_XEMPTY + 8 * buf, ((n >> 1) & 1) ^ 1);
-                if (gave_up(abort_flag)) return;     // what is in flight has to land before the CTA leaves: no further copies
+                if (!acquire(bars + R_XEMPTY + 8 * buf, ((n >> 1) & 1) ^ 1, abort_flag, P.status)) return;
                 if (one) bar_expect_tx(xf, nb * X_BLOCK);
                 if (one)
                     for (int c = 0; c < nb / 4; c++) tma_load_2d(sb + L.x + (buf * nb + 4 * c) * X_BLOCK, &tmX, c * 128, tt * NT, xf);
@@ -240,10 +239,9 @@ k_q8_gemm_res(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ C
                     // the places of a half are free when the last tile's MMAs of that half are complete
 #pragma unroll 1
                     for (int q = 0; q < 16; q++) {
-                        if ((q & 7) == 0) wait(bars + R_SEMPTY + q, (n & 1) ^ 1);
+                        if ((q & 7) == 0 && !acquire(bars + R_SEMPTY + q, (n & 1) ^ 1, abort_flag, P.status)) return;
                         const int l = brev4(q), two = l + 16 < nb;
                         const unsigned wf = bars + R_WFULL + 8 * q;
-                        if (gave_up(abort_flag)) return;
                         if (one) {
                             bar_expect_tx(wf, (1 + two) * W_BLOCK);
                             tma_load_2d(sb + l * W_BLOCK, &tmW, l * 32, rt * TM, wf);
@@ -542,7 +540,6 @@ k_q8_gemm_pair(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ 
 #pragma unroll 1
             for (int b = pair_lane(j); b < nb; b += 32) g(b);
     };
-    auto wait = [&](unsigned bar, unsigned parity) { bar_wait(bar_test(bar, parity), bar, parity, abort_flag, P.status); };
 
     if (warp >= 2 * EW) {
         asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(RES_AUX_REGS));
@@ -613,8 +610,7 @@ k_q8_gemm_pair(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ 
             bool any = false;
             auto write = [&]() {
                 const unsigned full = bars + P_FULL + 8 * s, wdst = sb + M::W + s * 4 * W_BLOCK, xdst = sb + M::X + s * 4 * X_BLOCK;
-                wait(bars + P_EMPTY + 8 * s, phase);
-                if (gave_up(abort_flag)) return;     // what is in flight has to land before the CTA leaves: no further copies
+                if (!acquire(bars + P_EMPTY + 8 * s, phase, abort_flag, P.status)) return;
                 if (one) {
                     bar_expect_tx(full, 4 * (W_BLOCK + X_BLOCK));
                     tma_load_2d(wdst, &tmW, held_b * 32, held_row, full);

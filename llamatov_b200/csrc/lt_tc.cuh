@@ -84,8 +84,14 @@ __device__ __forceinline__ void bar_wait(bool done, unsigned bar, unsigned parit
         atomicOr(status, LT_STATUS_WAIT_TIMEOUT);
     });
 }
-// for a whole warp: has a wait of the CTA run out of time?
-__device__ __forceinline__ bool gave_up(const volatile int* abort_flag) { return __any_sync(0xffffffffu, *abort_flag != 0); }
+// The wait of a whole warp for a place that it fills by bulk copies: false once a wait of the CTA has run out of time and the place is
+// not free.  No copy is begun then, since what is in flight has to land before the CTA leaves.  (The flag is looked at where the
+// place is not free at once: at every step it cost 28672 x 4096 x 32 3 %.)
+__device__ __forceinline__ bool acquire(unsigned bar, unsigned parity, volatile int* abort_flag, int* status) {
+    if (__all_sync(0xffffffffu, bar_test(bar, parity))) return true;
+    bar_wait(false, bar, parity, abort_flag, status);
+    return !__any_sync(0xffffffffu, *abort_flag != 0);
+}
 
 // One thread of a converged warp.  Roles whose single thread issues copies or MMAs run their loops as a warp and pick the
 // thread at the instruction: counters and descriptors then stay in uniform registers, which those instructions read.
