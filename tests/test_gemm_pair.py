@@ -89,3 +89,25 @@ def test_pair_gemm_unusual_scales(K):
         want, got = _gemm(Wq, Wd, Xq, Xd, M, K, T, 1), _gemm(Wq, wd, Xq, xd, M, K, T, 6)
         assert torch.equal(want.view(torch.int32), got.view(torch.int32)) and not torch.isfinite(want[0, 17])
     assert _lib.device_status() == set()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("M,K,T", [(4096, 14336, 256), (1200, 896, 900)])
+def test_pair_gemm_rows_with_an_infinite_scale(M, K, T):
+    """A row in 128 with an infinite scale, one column with an infinite scale: the bits of the 16-column tiles, in at most five times the
+    time (one thread per row and columns byte by byte took 67 times as long)."""
+    Wq, Wd, Xq, Xd = _operands(M, K, T, 4)
+
+    def us(variant):
+        ev = [torch.cuda.Event(enable_timing=True) for _ in range(6)]
+        for e in ev:
+            y = _gemm(Wq, Wd, Xq, Xd, M, K, T, variant)
+            e.record()
+        torch.cuda.synchronize()
+        return y, sorted(a.elapsed_time(b) for a, b in zip(ev, ev[1:]))[2]
+    plain = us(6)[1]
+    Wd[5::128, K // 64], Xd[T // 2, 1] = float("inf"), float("inf")
+    got, odd = us(6)
+    assert torch.equal(us(1)[0].view(torch.int32), got.view(torch.int32)) and not torch.isfinite(got[0, 5]) and torch.isfinite(got[0, 6])
+    assert odd < 5 * plain + 0.05, (plain, odd)
+    assert _lib.device_status() == set()
