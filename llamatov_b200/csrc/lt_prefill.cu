@@ -561,7 +561,7 @@ static int launch_attn_prefill_wide(const float* Q, int q_ld, const AttnSeqs& S,
 // cores: no SM holds 32 rows of scores beside the tiles, and nothing depends on Lmax.  A row's 64 softmax lanes are the 64 positions of
 // a tile, so the lane sums of the denominator stay in the registers of the threads that make the probabilities.  Bound by the operand reads (twice the clocks of the
 // multiply-adds) and issue slots of its two exact products of Lmax^2 / 2 x HD per head and by the uneven lengths of the rows.
-// 2048 positions: 14 heads on 2 of 64: 505 us with 16 rows, now 305; 32 heads on 8 of 128: 3273, now 1269.
+// 2048 positions: 14 heads on 2 of 64: 505 us with 16 rows, now 310; 32 heads on 8 of 128: 3273, now 1266.
 // (64 rows per CTA, 8 x 4 per thread: 444; the 448 CTAs are all resident at once and share the SMs unevenly.)
 constexpr int PB_TILE = 64;
 
@@ -671,9 +671,10 @@ k_attn_prefill_block(const float* __restrict__ Q, int q_ld, const __grid_constan
     // declared chain of every warp's greatest gives a score that the maximum reaches at least; what else may reach it (one or two of
     // a row, from the first two of a thread) is folded too.  Where a third may, or many do (rows of equal scores), or eps is no bound
     // (norms at the end of fp16 or beyond, or not finite), the blocked product finds the maxima.
-    // 2048 positions, us, with the blocked product alone and so: 14 heads of 64 349 and 305, 32 heads of 128 1549 and 1269; keys with
-    // a bias of three times their deviation 349 and 306, of twenty times 349 and 389, equal keys 350 and 418.  (bf16 needs a bound
-    // four times as wide; products in tf32: 406; candidates found by a second walk over K: 350.)
+    // 2048 positions, us, with the blocked product alone and so: 14 heads of 64 350 and 310, 32 heads of 128 1550 and 1266; with keys
+    // whose bias is three times their deviation 349 and 310, 1549 and 1282; eight times 349 and 328, 1550 and 1394; twenty times 350
+    // and 383, 1547 and 1549; equal keys 350 and 360, 1550 and 1547.  (bf16 needs a bound four times as wide; products in tf32:
+    // 406; candidates found by a second walk over K: 350.)
     float mx[MQ];
 #pragma unroll
     for (int i = 0; i < MQ; i++) mx[i] = -1e30f;
@@ -733,57 +734,74 @@ k_attn_prefill_block(const float* __restrict__ Q, int q_ld, const __grid_constan
             bad = bad || !(qn[i] < 1e14f);
             top[i][0] = top[i][1] = top[i][2] = -1e38f;
         }
-        for (int t0 = 0, buf = 0; t0 < Lmax; t0 += PB_TILE, buf ^= 1) {
-            if (t0 + PB_TILE < Lmax) {
-                copy_tile(K, t0 + PB_TILE, buf ? tk : tv);
-                asm volatile("cp.async.wait_group 1;" ::: "memory");
-            } else {
-                asm volatile("cp.async.wait_group 0;" ::: "memory");
-            }
-            __syncthreads();
-            const float* kt = (buf ? tv : tk) + (w * 16 + g) * ST + 4 * t4;
-            const bool edge = t0 + PB_TILE > L0 + r0 + 1 || nq < QT;
-            const int tp = t0 + w * 16 + 2 * t4 - (L0 + r0 + g);
+        float kg = 0.0f;                         // norm of a key of the last tile
+        int t0 = 0, buf = 0;
+#pragma unroll 1
+        for (int end = 2 * PB_TILE < Lmax ? 2 * PB_TILE : Lmax;; end = Lmax) {
+#pragma unroll 1
+            for (; t0 < end; t0 += PB_TILE, buf ^= 1) {
+                if (t0 + PB_TILE < Lmax) {
+                    copy_tile(K, t0 + PB_TILE, buf ? tk : tv);
+                    asm volatile("cp.async.wait_group 1;" ::: "memory");
+                } else {
+                    asm volatile("cp.async.wait_group 0;" ::: "memory");
+                }
+                __syncthreads();
+                const float* kt = (buf ? tv : tk) + (w * 16 + g) * ST + 4 * t4;
+                const bool edge = t0 + PB_TILE > L0 + r0 + 1 || nq < QT;
+                const int tp = t0 + w * 16 + 2 * t4 - (L0 + r0 + g);
 #pragma unroll
-            for (int y = 0; y < 2; y++) {        // eight positions
-                float c[2][4], k2 = 0.0f;
-#pragma unroll
-                for (int x = 0; x < 2; x++)
-#pragma unroll
-                    for (int e = 0; e < 4; e++) c[x][e] = 0.0f;
-#pragma unroll
-                for (int cc = 0; cc < HD / 16; cc++) {
-                    const float4 k = *(const float4*)(kt + y * 8 * ST + 16 * cc);
-                    k2 += k.x * k.x + k.y * k.y + k.z * k.z + k.w * k.w;
-                    const unsigned k0 = fp16(k.x, k.y), k1 = fp16(k.z, k.w);
+                for (int y = 0; y < 2; y++) {        // eight positions
+                    float c[2][4], k2 = 0.0f;
 #pragma unroll
                     for (int x = 0; x < 2; x++)
-                        asm("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
-                            : "+f"(c[x][0]), "+f"(c[x][1]), "+f"(c[x][2]), "+f"(c[x][3])
-                            : "r"(qa[cc][x][0][0]), "r"(qa[cc][x][1][0]), "r"(qa[cc][x][0][1]), "r"(qa[cc][x][1][1]), "r"(k0), "r"(k1));
-                }
-                k2 += __shfl_xor_sync(0xffffffffu, k2, 1);
-                k2 += __shfl_xor_sync(0xffffffffu, k2, 2);
-                bad = bad || !(k2 < 4e9f);
-                const float kg = sqrtf(k2) + 0x1p-12f;           // of position g; the products are those of positions 2 t4 and 2 t4 + 1
-                const float kn[2] = {__shfl_sync(0xffffffffu, kg, 8 * t4), __shfl_sync(0xffffffffu, kg, 8 * t4 + 4)};
 #pragma unroll
-                for (int x = 0; x < 2; x++)
+                        for (int e = 0; e < 4; e++) c[x][e] = 0.0f;
 #pragma unroll
-                    for (int e = 0; e < 4; e++) {
-                        const int i = 2 * x + (e >> 1);
-                        float v = __fmaf_rn(c[x][e], scale, __fmaf_rn(qn[i], kn[e & 1], 1e-37f));
-                        if (edge && !(tp + 8 * y + (e & 1) <= 8 * i && g + 8 * i < nq)) v = -1e38f;
-                        v = __int_as_float((__float_as_int(v) & ~0x1fff) | (t0 / PB_TILE * 4 + 2 * y + (e & 1)));
-                        float(&a)[3] = top[i];
-                        const float d0 = fminf(a[0], v);
-                        a[0] = fmaxf(a[0], v);
-                        const float d1 = fminf(a[1], d0);
-                        a[1] = fmaxf(a[1], d0);
-                        a[2] = fmaxf(a[2], d1);
+                    for (int cc = 0; cc < HD / 16; cc++) {
+                        const float4 k = *(const float4*)(kt + y * 8 * ST + 16 * cc);
+                        k2 += k.x * k.x + k.y * k.y + k.z * k.z + k.w * k.w;
+                        const unsigned k0 = fp16(k.x, k.y), k1 = fp16(k.z, k.w);
+#pragma unroll
+                        for (int x = 0; x < 2; x++)
+                            asm("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
+                                : "+f"(c[x][0]), "+f"(c[x][1]), "+f"(c[x][2]), "+f"(c[x][3])
+                                : "r"(qa[cc][x][0][0]), "r"(qa[cc][x][1][0]), "r"(qa[cc][x][0][1]), "r"(qa[cc][x][1][1]), "r"(k0), "r"(k1));
                     }
+                    k2 += __shfl_xor_sync(0xffffffffu, k2, 1);
+                    k2 += __shfl_xor_sync(0xffffffffu, k2, 2);
+                    bad = bad || !(k2 < 4e9f);
+                    kg = sqrtf(k2) + 0x1p-12f;       // of position g; the products are those of positions 2 t4 and 2 t4 + 1
+                    const float kn[2] = {__shfl_sync(0xffffffffu, kg, 8 * t4), __shfl_sync(0xffffffffu, kg, 8 * t4 + 4)};
+#pragma unroll
+                    for (int x = 0; x < 2; x++)
+#pragma unroll
+                        for (int e = 0; e < 4; e++) {
+                            const int i = 2 * x + (e >> 1);
+                            float v = __fmaf_rn(c[x][e], scale, __fmaf_rn(qn[i], kn[e & 1], 1e-37f));
+                            if (edge && !(tp + 8 * y + (e & 1) <= 8 * i && g + 8 * i < nq)) v = -1e38f;
+                            v = __int_as_float((__float_as_int(v) & ~0x1fff) | (t0 / PB_TILE * 4 + 2 * y + (e & 1)));
+                            float(&a)[3] = top[i];
+                            const float d0 = fminf(a[0], v);
+                            a[0] = fmaxf(a[0], v);
+                            const float d1 = fminf(a[1], d0);
+                            a[1] = fmaxf(a[1], d0);
+                            a[2] = fmaxf(a[2], d1);
+                        }
+                }
+                __syncthreads();                     // the tile may be replaced
             }
-            __syncthreads();                     // the tile may be replaced
+            if (end == Lmax) break;
+            // Keys much alike, beside their lengths, leave too many in the end.  Where a 32nd of the threads have a third of their eight
+            // positions so far within reach of the warp's first (one of a thread's rows is asked; all four cost 2 us of code), the
+            // search ends here, and what it took is a few per cent.
+            float v = fmaxf(top[0][0], __shfl_xor_sync(0xffffffffu, top[0][0], 1));
+            v = fmaxf(v, __shfl_xor_sync(0xffffffffu, v, 2));
+            const bool near = bad || (top[0][2] > -9e37f && top[0][2] >= v - 2.0f * qn[0] * kg);
+            if (__syncthreads_count(near) >= PB_THREADS / 32) {
+                bad = true;
+                break;
+            }
         }
         auto position = [&](float v) {
             const int place = __float_as_int(v) & 0x1fff;
@@ -819,6 +837,7 @@ k_attn_prefill_block(const float* __restrict__ Q, int q_ld, const __grid_constan
 #pragma unroll
             for (int i = 0; i < MQ; i++) mx[i] = fmaxf(mx[i], __int_as_float(ordered(mk[m * MQ + i])));
         } else {
+            asm volatile("cp.async.wait_group 0;" ::: "memory");     // a tile may be on its way to where the first one goes
             copy_tile(K, 0, tk);
         }
     }
