@@ -42,51 +42,78 @@ def _blocks(seed):
 
 
 def _expected(x):
-    """Bytes and scales by the definition, in fp32 divisions; None for blocks with NaNs."""
+    """Bytes and scales by the definition, in fp32 divisions.  The greatest value comes by a butterfly over the block, so that beside
+    NaNs, which compare false, every element has its own; the block's scale is the first element's."""
     with np.errstate(all="ignore"):
-        amax = np.abs(x).max(1)
+        amax = np.abs(x)
+        for s in (16, 8, 4, 2, 1):
+            other = amax[:, np.arange(32) ^ s]
+            amax = np.where(other > amax, other, amax)
         d = np.where(amax > 0, amax / np.float32(127), np.float32(1)).astype(np.float32).astype(np.float16)
-        q = np.rint(x / d.astype(np.float32)[:, None])
+        q = np.rint(x / d.astype(np.float32))
         q = np.where(np.isnan(q), 0, np.clip(q, -127, 127)).astype(np.int8)
-    return q, d.view(np.uint16)
+    return q, d[:, 0].view(np.uint16)
 
 
-@pytest.mark.parametrize("rows", [1, 40])     # a lane per value, four values per thread
-def test_quantiser_rounds_like_the_divisions(rows):
-    x = _blocks(rows)
-    x = x[:len(x) // rows * rows].reshape(rows, -1) if rows > 1 else x.reshape(1, -1)
-    if rows == 1:
-        x = x[:, :32 * 2000]                  # few blocks: the form with a lane per value
-        x[:, -32 * 64:] = _blocks(1)[-64:].reshape(1, -1)
-    K = x.shape[1]
-    dx = torch.from_numpy(np.ascontiguousarray(x)).cuda()
-    xq, xd = torch.empty(x.shape, dtype=torch.int8, device="cuda"), torch.empty((rows, K // 32), dtype=torch.int16, device="cuda")
+@pytest.mark.parametrize("per_call", [8000, 1 << 20])     # a lane per value (few blocks), four values per thread
+def test_quantiser_rounds_like_the_divisions(per_call):
+    blocks = _blocks(1)
+    assert len(blocks) > 148 * 64 * 2 and np.isnan(blocks).any(1).sum() > 8
     st = torch.cuda.current_stream().cuda_stream
-    _lib.call("lt_quant_q8", dx.data_ptr(), xq.data_ptr(), xd.data_ptr(), K, rows, st)
-    b = x.reshape(-1, 32)
-    q, d = _expected(b)
-    ok = ~np.isnan(b).any(1)
-    assert ok.sum() > 1000
-    assert np.array_equal(xd.cpu().numpy().view(np.uint16).reshape(-1)[ok], d[ok])
-    assert np.array_equal(xq.cpu().numpy().reshape(-1, 32)[ok], q[ok])
+    for i in range(0, len(blocks), per_call):
+        b = np.ascontiguousarray(blocks[i:i + per_call])
+        dx = torch.from_numpy(b).cuda()
+        xq, xd = torch.empty(b.shape, dtype=torch.int8, device="cuda"), torch.empty(len(b), dtype=torch.int16, device="cuda")
+        _lib.call("lt_quant_q8", dx.data_ptr(), xq.data_ptr(), xd.data_ptr(), b.size, 1, st)
+        q, d = _expected(b)
+        assert np.array_equal(xd.cpu().numpy().view(np.uint16), d)
+        assert np.array_equal(xq.cpu().numpy(), q)
+
+
+def _behind_the_norm(Wq, Wd, x, w, eps):
+    """(norm, quantiser and projection one by one; the projection that does all three; the norm's output)"""
+    M, K = Wq.shape
+    st = torch.cuda.current_stream().cuda_stream
+    n = torch.empty(K, device="cuda")
+    xq, xd = torch.empty(K, dtype=torch.int8, device="cuda"), torch.empty(K // 32, dtype=torch.int16, device="cuda")
+    y0, y1 = torch.empty(M, device="cuda"), torch.empty(M, device="cuda")
+    _lib.call("lt_rmsnorm", x.data_ptr(), w.data_ptr(), n.data_ptr(), 1, K, eps, st)
+    _lib.call("lt_quant_q8", n.data_ptr(), xq.data_ptr(), xd.data_ptr(), K, 1, st)
+    _lib.call("lt_q8_gemv", Wq.data_ptr(), Wd.data_ptr(), xq.data_ptr(), xd.data_ptr(), None, y0.data_ptr(), M, K, 1, st)
+    _lib.call("lt_rmsnorm_q8_gemv", Wq.data_ptr(), Wd.data_ptr(), x.data_ptr(), w.data_ptr(), eps, None, y1.data_ptr(), M, K, st)
+    return y0.view(torch.int32), y1.view(torch.int32), n
+
+
+def _matrix(M, K, g):
+    return (torch.randint(-127, 128, (M, K), generator=g, dtype=torch.int8, device="cuda"),
+            (torch.rand((M, K // 32), generator=g, device="cuda") * 0.02).half())
 
 
 def test_quantiser_behind_the_norm_rounds_like_the_separate_one():
-    """The projection that normalises and quantises for itself against norm, quantiser and projection: the same bits, NaNs
-    (which every value of a row sees) included."""
-    K, M, st = 1152, 64, torch.cuda.current_stream().cuda_stream
-    g = torch.Generator(device="cuda").manual_seed(4)
-    Wq = torch.randint(-127, 128, (M, K), generator=g, dtype=torch.int8, device="cuda")
-    Wd = (torch.rand((M, K // 32), generator=g, device="cuda") * 0.02).half()
+    """The projection that normalises and quantises for itself against norm, quantiser and projection: the same bits, also for
+    rows with a NaN or an infinity, whose norm every value sees."""
+    K, g = 1152, torch.Generator(device="cuda").manual_seed(4)
+    Wq, Wd = _matrix(64, K, g)
     w = torch.randn(K, generator=g, device="cuda")
-    for scale in (1.0, 1e-12, 3e4):
+    for scale, odd in ((1.0, 0.0), (1e-12, 0.0), (3e4, 0.0), (1.0, float("nan")), (1.0, float("inf"))):
         x = torch.randn(K, generator=g, device="cuda") * scale
-        n = torch.empty(K, device="cuda")
-        xq, xd = torch.empty(K, dtype=torch.int8, device="cuda"), torch.empty(K // 32, dtype=torch.int16, device="cuda")
-        y0, y1 = torch.empty(M, device="cuda"), torch.empty(M, device="cuda")
-        _lib.call("lt_rmsnorm", x.data_ptr(), w.data_ptr(), n.data_ptr(), 1, K, 1e-5, st)
-        _lib.call("lt_quant_q8", n.data_ptr(), xq.data_ptr(), xd.data_ptr(), K, 1, st)
-        _lib.call("lt_q8_gemv", Wq.data_ptr(), Wd.data_ptr(), xq.data_ptr(), xd.data_ptr(), None, y0.data_ptr(), M, K, 1, st)
-        _lib.call("lt_rmsnorm_q8_gemv", Wq.data_ptr(), Wd.data_ptr(), x.data_ptr(), w.data_ptr(), 1e-5, None, y1.data_ptr(), M, K, st)
-        assert torch.equal(y0.view(torch.int32), y1.view(torch.int32))
+        if odd:
+            x[77] = odd
+        y0, y1, _ = _behind_the_norm(Wq, Wd, x, w, 1e-5)
+        assert torch.equal(y0, y1)
+    assert _lib.device_status() == set()
+
+
+def test_quantiser_behind_the_norm_at_the_boundaries():
+    """The same where the norm's output is its weight (rows of ones, no epsilon): the blocks above, whose values lie at the middles of
+    integers and whose scales at the middles of fp16, 36 a call."""
+    K, g = 1152, torch.Generator(device="cuda").manual_seed(5)
+    Wq, Wd = _matrix(64, K, g)
+    blocks = _blocks(2)
+    blocks = blocks[np.isfinite(blocks).all(1)]
+    x = torch.ones(K, device="cuda")
+    for i in range(0, len(blocks) - 36, len(blocks) // 300):
+        w = torch.from_numpy(blocks[i:i + 36].reshape(-1)).cuda()
+        y0, y1, n = _behind_the_norm(Wq, Wd, x, w, 0.0)
+        assert torch.equal(n, w) and torch.equal(y0, y1)
     assert _lib.device_status() == set()
