@@ -768,8 +768,9 @@ extern "C" int lt_attn_decode_batch(const float* Q, int q_ld, const float* K, co
         e = launch_chained(k_attn_softmax, dim3(nh, B), dim3(BT), (size_t)max_seq * sizeof(float), s, S, s_ld, lens, Z, nh,
                            max_seq);
     if (e == cudaSuccess) {
-        // A warp per 64 elements needs CTAs enough, and rows long enough for its ring; with one query head per KV head it has the
-        // other form's CTAs and longer reads.  32 heads on 8 of 128, 1024 positions, 8 sequences (128 CTAs) 41 us against 30, 12
+        // A warp per 64 elements has half of the other form's CTAs; it needs CTAs enough, and rows long enough for its ring.  With one
+        // query head per KV head both forms have one warp a CTA and the longer reads win throughout (the whole attention, 2, 8 and
+        // 32 KV heads, 1 to 32 sequences, 40 to 2000 positions: heads of 64 0.59 to 1.00 of the time, of 128 0.58 to 1.00).  32 heads on 8 of 128, 1024 positions, 8 sequences (128 CTAs) 41 us against 30, 12
         // (192) 46.8, 47.7, 24 59, 64, 32 67, 76; 500 positions 12 sequences 28.2, 27.8, 24 35, 37; 100 positions 32 sequences
         // 15.8, 15.3.  8 heads on 8 of 128, 1024 positions: 24 us against 28 for one sequence, 37 against 62 for 16.
         const long ctas = (long)(hd / 64) * nkv * B;

@@ -164,8 +164,9 @@ __device__ __forceinline__ float q8_reciprocal(float d) {   // relative error be
     return r;
 }
 // r = q8_reciprocal(d).  |v| <= amax bounds the quotient by 191 (d is rounded, at worst from 1.5 to 1 unit of the smallest fp16),
-// so t is off by less than 6e-5 and a t that is 1e-4 or more from the middle of two integers rounds like the quotient.  A block
-// with a NaN has d = 1, where t = v; NaN and infinite t divide.
+// so t is off by less than 6e-5 and a t that is 1e-4 or more from the middle of two integers rounds like the quotient.  In a
+// block with a NaN either d = 1, where t is v within 2^-22 of it and what lies beyond 191 is clamped, or amax is the element's own
+// (the greatest of some of the block's values, its own among them).  NaN and infinite t divide.
 __device__ __forceinline__ int q8_value(float v, float d, float r) {
     const float t = __fmul_rn(v, r);
     float n = rintf(t);

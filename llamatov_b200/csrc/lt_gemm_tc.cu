@@ -538,10 +538,11 @@ static int choose_split(int M, int K, int T, int sms, int room2, int room4) {
     return 1 << best;
 }
 
-// The 32-column tiles of lt_gemm_pair.cu where they are faster by more than their times scatter.  Over the 1187 measured shapes
-// the choice is within 0.5 % of the best on average and none is slower than without it by more than 3 %.  Few columns of a
-// small matrix stay here: the other kernels' first tile comes 4 us later (896 x 896 x 64 6.7 us, 9.3; x 2048 31, 22;
-// 4096 x 4096 x 64 18.3, 21.4; 28672 x 4096 x 32 61, 45).
+// The 32-column tiles of lt_gemm_pair.cu where they are faster by more than their times scatter.  Over 292 shapes (15 matrices
+// from 128 x 512 to 128256 x 4096, 9 to 2048 columns) the chosen form takes 0.1 % more than the better one on average, at most 9 %
+// (1024 x 640 x 512, which stays here at 10.0 us against 9.2), and never more than 2 % over the form here.  Few columns of a
+// small matrix stay here: the other kernels' first tile comes 3 us later (896 x 896 x 64 6.8 us, 9.6; x 2048 30, 22;
+// 4096 x 4096 x 64 17.1, 20.7; 28672 x 4096 x 32 61, 43).
 static bool choose_pair(int M, int K, int T, int sms, int room2, int room4) {
     const int nb = K / 32, S = choose_split(M, K, T, sms, room2, room4);
     const long rooms = S == 4 ? room4 : (S == 2 ? room2 : sms), tiles = (long)((M + TM - 1) / TM) * ((T + 15) / 16);

@@ -561,9 +561,11 @@ static int launch_attn_prefill_wide(const float* Q, int q_ld, const AttnSeqs& S,
 // cores: no SM holds 32 rows of scores beside the tiles, and nothing depends on Lmax.  A row's 64 softmax lanes are the 64 positions of
 // a tile, so the lane sums of the denominator stay in the registers of the threads that make the probabilities.  Bound by the operand reads (twice the clocks of the
 // multiply-adds) and issue slots of its two exact products of Lmax^2 / 2 x HD per head and by the uneven lengths of the rows.
-// 2048 positions: 14 heads on 2 of 64: 505 us with 16 rows, now 310; 32 heads on 8 of 128: 3273, now 1266.
+// 2048 positions: 14 heads on 2 of 64: 505 us with 16 rows, now 314; 32 heads on 8 of 128: 3273, now 1273.
 // (64 rows per CTA, 8 x 4 per thread: 444; the 448 CTAs are all resident at once and share the SMs unevenly.)
 constexpr int PB_TILE = 64;
+constexpr int PREFILL_MAXT = 12000;      // positions that the entry points take
+static_assert(PREFILL_MAXT <= PB_TILE * 2048, "a position's place within its thread has 13 bits");
 
 template <int HD, int QT>
 struct PrefillBlock {
@@ -671,15 +673,15 @@ k_attn_prefill_block(const float* __restrict__ Q, int q_ld, const __grid_constan
     // declared chain of every warp's greatest gives a score that the maximum reaches at least; what else may reach it (one or two of
     // a row, from the first two of a thread) is folded too.  Where a third may, or many do (rows of equal scores), or eps is no bound
     // (norms at the end of fp16 or beyond, or not finite), the blocked product finds the maxima.
-    // 2048 positions, us, with the blocked product alone and so: 14 heads of 64 350 and 310, 32 heads of 128 1550 and 1266; with keys
-    // whose bias is three times their deviation 349 and 310, 1549 and 1282; eight times 349 and 328, 1550 and 1394; twenty times 350
-    // and 383, 1547 and 1549; equal keys 350 and 360, 1550 and 1547.  (bf16 needs a bound four times as wide; products in tf32:
+    // 2048 positions, us, with the blocked product alone and so: 14 heads of 64 350 and 314, 32 heads of 128 1550 and 1273; with keys
+    // whose bias is three times their deviation 349 and 314, 1549 and 1288; eight times 349 and 331, 1550 and 1401; twenty times 350
+    // and 369, 1547 and 1558; equal keys 350 and 350, 1550 and 1558.  (bf16 needs a bound four times as wide; products in tf32:
     // 406; candidates found by a second walk over K: 350.)
     float mx[MQ];
 #pragma unroll
     for (int i = 0; i < MQ; i++) mx[i] = -1e30f;
-    bool blocked = true;
-    if (Lmax <= PB_TILE * 2048) {
+    bool blocked;
+    {
         static_assert(QT == 32 && PB_THREADS == 128 && PB_TILE == 64, "a warp takes 16 positions of a tile for 32 rows");
         constexpr int NCAND = 2 * PB_THREADS;    // one for each warp and row, as many others
         const int w = tid >> 5, g = (tid & 31) >> 2, t4 = tid & 3;
@@ -1007,7 +1009,8 @@ static int pick_attn_prefill_rows(const float* Q, int q_ld, const AttnSeqs& S, i
     if (nrows >= 32 && aligned) {
         // 32 rows per CTA from two CTAs (heads of 64) or 9/4 (heads of 128) for each SM on; below, smaller tiles fill the SMs
         // better.  us with 16 and with 32 rows per CTA: 14 heads of 64, 333 rows (154 CTAs) 31 and 36, 500 (224) 52 and 60, 600 (266)
-        // 67 and 62, 700 (308) 84 and 79, 850 (378) 115 and 97; of 128, 16 heads, 600 rows (304) 121 and 125, 32 heads, 300 rows
+        // 67 and 62, 700 (308) 84 and 79, 850 (378) 115 and 97 (with
+        // equal keys, whose maxima the blocked product finds, 700 rows 91, 850 rows 113); of 128, 16 heads, 600 rows (304) 121 and 125, 32 heads, 300 rows
         // (320) 74 and 67, 400 behind 700 positions (416) 358 and 346.
         if ((long)((nrows + 31) / 32) * nh * nseq * 4 >= (HD == 64 ? 8L : 9L) * sm_count())
             return launch_attn_prefill_block<HD, 32>(Q, q_ld, S, nseq, OUT, out_ld, nh, nkv, scale, nrows, maxt, s);
@@ -1126,7 +1129,7 @@ extern "C" int lt_attn_prefill(const float* Q, int q_ld, const float* K, const f
     LT_REQUIRE(Q && K && V && len && OUT, "lt_attn_prefill: null pointer");
     LT_REQUIRE(hd == 64 || hd == 128, "lt_attn_prefill: hd=%d (64 and 128 are built)", hd);
     LT_REQUIRE(nh > 0 && nkv > 0 && nh % nkv == 0, "lt_attn_prefill: nh=%d must be a positive multiple of nkv=%d", nh, nkv);
-    LT_REQUIRE(nrows > 0 && maxt >= nrows && maxt <= 12000, "lt_attn_prefill: nrows=%d maxt=%d (maxt in nrows..12000)", nrows, maxt);
+    LT_REQUIRE(nrows > 0 && maxt >= nrows && maxt <= PREFILL_MAXT, "lt_attn_prefill: nrows=%d maxt=%d (maxt in nrows..%d)", nrows, maxt, PREFILL_MAXT);
     LT_REQUIRE(q_ld >= nh * hd && out_ld >= nh * hd && q_ld % 4 == 0, "lt_attn_prefill: q_ld=%d out_ld=%d", q_ld, out_ld);
     LT_REQUIRE(out_ld % 2 == 0 && (reinterpret_cast<uintptr_t>(OUT) & 7u) == 0 && (reinterpret_cast<uintptr_t>(V) & 7u) == 0,
                "lt_attn_prefill: OUT and V must be 8-byte aligned, out_ld even");
@@ -1152,7 +1155,7 @@ extern "C" int lt_attn_prefill_rows(const float* Q, int q_ld, const lt_row_seqs*
         ok = ok && aligned16(S.k[b]) && (reinterpret_cast<uintptr_t>(S.v[b]) & 7u) == 0;
     }
     cudaStream_t s = (cudaStream_t)stream;
-    if (ok && maxt <= 12000) {
+    if (ok && maxt <= PREFILL_MAXT) {
         rc = hd == 64 ? pick_attn_prefill_rows<64>(Q, q_ld, S, B, OUT, out_ld, nh, nkv, scale, T, maxt, s)
                       : pick_attn_prefill_rows<128>(Q, q_ld, S, B, OUT, out_ld, nh, nkv, scale, T, maxt, s);
         if (rc != LT_ERR_UNSUPPORTED) return rc;
