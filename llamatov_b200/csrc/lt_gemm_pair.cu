@@ -14,7 +14,7 @@
 // What bounded the 16-column tiles (9728 x 896 x 2048, 264 us): 1070 clocks per 8192 block sums, of which 256 are shared-memory
 // reads of activation scales (a broadcast 16-byte read still writes 512 bytes of registers), the rest uncoalesced loads of
 // weight scales and hand-overs.  Here 480 clocks (139 us; 28672 x 4096 x 512 683 -> 379 us, 4096 x 14336 x 512 330 -> 228 us):
-// the epilogue's issue slots, 70 % busy; conversions and fp32 pipes have 128 of the 480 to do, the MMAs 130.
+// the epilogue's issue slots, 68 to 70 % busy by the counters; by count, conversions and fp32 pipes have 128 of the 480 to do, the MMAs 130.
 // An epilogue thread is one row x 16 columns; a copy of its sums or a poll costs as much as a fold, and its waits are as long
 // as its arithmetic, so two sets of eight epilogue warps work on different l (the even and the odd ones).
 // Two kernels: k_q8_gemm_res for rows of 512 to 896 values, k_q8_gemm_pair for any; lt_q8_gemm_tc chooses between them and the

@@ -1009,9 +1009,9 @@ static int pick_attn_prefill_rows(const float* Q, int q_ld, const AttnSeqs& S, i
     if (nrows >= 32 && aligned) {
         // 32 rows per CTA from two CTAs (heads of 64) or 9/4 (heads of 128) for each SM on; below, smaller tiles fill the SMs
         // better.  us with 16 and with 32 rows per CTA: 14 heads of 64, 333 rows (154 CTAs) 31 and 36, 500 (224) 52 and 60, 600 (266)
-        // 67 and 62, 700 (308) 84 and 79, 850 (378) 115 and 97 (with
-        // equal keys, whose maxima the blocked product finds, 700 rows 91, 850 rows 113); of 128, 16 heads, 600 rows (304) 121 and 125, 32 heads, 300 rows
-        // (320) 74 and 67, 400 behind 700 positions (416) 358 and 346.
+        // 67 and 62, 700 (308) 84 and 79, 850 (378) 115 and 97 (with equal keys, whose maxima the blocked product finds, 700 rows 91, 850
+        // rows 113); of 128, 16 heads, 600 rows (304) 121 and 125, 32 heads, 300 rows (320) 74 and 67, 400 behind 700 positions (416)
+        // 358 and 346.
         if ((long)((nrows + 31) / 32) * nh * nseq * 4 >= (HD == 64 ? 8L : 9L) * sm_count())
             return launch_attn_prefill_block<HD, 32>(Q, q_ld, S, nseq, OUT, out_ld, nh, nkv, scale, nrows, maxt, s);
         // ... where the score rows of 16 queries fit one SM beside double-buffered tiles
