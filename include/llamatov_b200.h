@@ -280,7 +280,8 @@ int lt_decode_pdl_num_parts(void);
  * lt_attn_prefill       k_attn_decode_masked (dev_residency.py:1955-2010) for the nrows rows just
  *                       appended: *len is the length after the append, row r is the query at position
  *                       *len - nrows + r and sees the positions up to and including its own.
- *                       maxt >= *len bounds the shared-memory score rows (<= 12000). */
+ *                       maxt >= *len bounds the shared-memory score rows (<= 12000).  A row none of whose
+ *                       scores reaches -1e30 (the score of masked positions) is zeros. */
 int lt_embed_q8_rows(const int8_t* Wq, const uint16_t* Wd, const int* toks, float* out, int E, int V,
                      int nrows, void* stream);
 int lt_rope_rows(float* X, int ld, const int* pos0, int nrows, int n_head, int hd, float theta, void* stream);

@@ -156,6 +156,10 @@ __global__ void k_silu_mul_quant_rows_lane(const float* __restrict__ G, const fl
 constexpr int PF_THREADS = 256;
 constexpr int PF_KTILE = 128;            // K rows staged per tile: two threads per position
 
+// What a row divides by.  A row none of whose scores reaches -1e30, the score of masked positions in the declared order (infinite and huge
+// queries), has only zeros as probabilities; the declared kernel then counts its masked positions and returns zeros.
+__device__ __forceinline__ float denominator(float z) { return z == 0.0f ? 1.0f : z; }
+
 // The sequences of a launch.  One: its length on the device; several: their lengths after the append, from the host.  Together
 // short prompts fill the SMs with blocks of 32 rows (three of 333: 87 us one after the other with 16 rows, 55 together).
 struct AttnSeqs {
@@ -265,7 +269,7 @@ k_attn_prefill(const float* __restrict__ Q, int q_ld, const float* __restrict__ 
         if (l64 < 32) {
             float v = __fadd_rn(red[qi * 64 + l64], red[qi * 64 + l64 + 32]);
             v = warp_tree_sum(v);
-            if (l64 == 0) zs[qi] = v;
+            if (l64 == 0) zs[qi] = denominator(v);
         }
         __syncthreads();
     }
@@ -459,7 +463,7 @@ k_attn_prefill_wide(const float* __restrict__ Q, int q_ld, const __grid_constant
         if (l64 < 32) {
             float v = __fadd_rn(red[qi * 64 + l64], red[qi * 64 + l64 + 32]);
             v = warp_tree_sum(v);
-            if (l64 == 0) zs[qi] = v;
+            if (l64 == 0) zs[qi] = denominator(v);
         }
         __syncthreads();
     }
@@ -950,7 +954,7 @@ k_attn_prefill_block(const float* __restrict__ Q, int q_ld, const __grid_constan
     __syncthreads();
     for (int r = tid >> 5; r < QT; r += PB_THREADS / 32) {
         const float v = warp_tree_sum(__fadd_rn(ps[r * PST + (tid & 31)], ps[r * PST + (tid & 31) + 32]));
-        if ((tid & 31) == 0) zs[r] = v;
+        if ((tid & 31) == 0) zs[r] = denominator(v);
     }
     __syncthreads();
 #pragma unroll

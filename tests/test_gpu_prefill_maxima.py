@@ -84,3 +84,27 @@ def test_row_maxima_where_sixteen_bits_round_to_one_side(name, hd, nh, nkv, T, L
         want = attend(Q[r:], K, V, n, L0 + r + n, hd, nh, nkv, scale)
         assert torch.equal(got[r:r + n], want), (name, r)
     assert torch.isfinite(got).all() and _lib.device_status() == set()
+
+
+@pytest.mark.parametrize("hd,nh,nkv,T,L0", [(64, 14, 2, 700, 3), (128, 16, 4, 832, 0), (64, 14, 2, 333, 0), (64, 14, 2, 20, 9)])
+def test_rows_whose_scores_are_all_below_the_mask(hd, nh, nkv, T, L0):
+    """Scores of minus infinity, and below -1e30, throughout a row: zeros, as from the one-token kernel, in every form (32 rows per
+    CTA, 16, fewer) and wherever in its tile the row is."""
+    g = torch.Generator(device="cuda").manual_seed(T)
+    L = L0 + T
+    Q, K, V = (torch.randn((n, w, hd), device="cuda", generator=g) for n, w in ((T, nh), (L, nkv), (L, nkv)))
+    K[..., 0] = 1 + K[..., 0].abs()
+    rows = [r for r in (0, 5, 7, 15, 16, 31, 33, T - 1) if r < T]
+    for i, r in enumerate(rows):
+        Q[r] = 0
+        Q[r, :, 0] = (-INF, -1e38)[i % 2]
+    Q, K = Q.reshape(T, -1), K.reshape(L, -1)
+    got = attend(Q, K, V, T, L, hd, nh, nkv, 0.125)
+    assert (got[rows] == 0).all() and torch.isfinite(got).all()
+    one, Kr, Vr = torch.empty(nh * hd, device="cuda"), torch.cat([K, K[:1]]), torch.cat([V, V[:1]])      # room for one more position
+    for r in rows + [T // 2]:
+        ln = torch.tensor([L0 + r + 1], dtype=torch.int32, device="cuda")
+        _lib.call("lt_attn_decode_masked", Q[r].data_ptr(), Kr.data_ptr(), Vr.data_ptr(), ln.data_ptr(), one.data_ptr(), hd, nh, nkv, 0.125, L + 1,
+                  torch.cuda.current_stream().cuda_stream)
+        assert torch.equal(one, got[r]), r
+    assert _lib.device_status() == set()
